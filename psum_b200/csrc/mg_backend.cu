@@ -34,6 +34,7 @@
 #include "mg_backend.hpp"
 #include "mg_host.hpp"
 #include "mg_kernels.cuh"
+#include "mg_persist.cuh"
 
 namespace psum_b200 {
 
@@ -48,6 +49,8 @@ constexpr int kNormBlocks = 444;   // 3 x 148 SMs: fixed grid -> fixed reduction
 template <class T>
 struct DevStencil {
     StencilDev<T> view{};
+    PersistStencil<T> persist{};   // the operator as the one-kernel solve reads it
+    DevBuf<unsigned char> rows;    // its exception words, coefficients and flags, one buffer
     DevBuf<uint32_t> mask, mask_prefix;
     DevBuf<int> exc_ptr, exc_col;
     DevBuf<T> exc_val;
@@ -83,6 +86,62 @@ struct DevStencil {
         view.exc_ptr = exc_ptr.p;
         view.exc_col = exc_col.p;
         view.exc_val = exc_val.p;
+        upload_persist(op, s);
+    }
+
+    // The stencil's shape, and every exception row as coefficients on the
+    // shape's taps.  A row whose columns do not ascend with the taps (it
+    // wraps around a face) would be summed in another order there: it keeps
+    // its column list.
+    void upload_persist(const StencilOp& op, cudaStream_t s) {
+        persist = PersistStencil<T>{};
+        persist.s = view;
+        for (int ns : {3, 5, 7, 9, 27}) {
+            bool same = ns == op.ns;
+            for (int t = 0; t < ns && same; ++t)
+                for (int a = 0; a < 3; ++a) same = same && op.delta[t][a] == shape_tap(ns, t, a);
+            for (int a = 0; a < 3; ++a) same = same && op.dims[a] != 2;   // -1 and +1 would be the same neighbour
+            if (ns == 3 || ns == 5 || ns == 9) same = same && op.dims[2] == 1 && (ns != 3 || op.dims[1] == 1);
+            if (same) persist.shape = ns;
+        }
+        if (!persist.shape || !exceptions) return;
+        std::vector<uint2> w(op.mask.size());
+        for (size_t q = 0; q < w.size(); ++q) w[q] = make_uint2(op.mask[q], op.mask_prefix[q]);
+        std::vector<T> c((size_t)exceptions * persist.shape, T(0));
+        std::vector<uint8_t> list((size_t)exceptions, 0);
+        bool any_list = false;
+        for (long long q = 0; q < exceptions; ++q) {
+            const int r = op.exc_rows[q];
+            const int rc[3] = {r / (op.dims[1] * op.dims[2]), r / op.dims[2] % op.dims[1], r % op.dims[2]};
+            int t = -1;
+            bool ok = true;
+            for (int e = op.exc_ptr[q]; e < op.exc_ptr[q + 1] && ok; ++e) {
+                int found = -1;
+                for (int u = t + 1; u < persist.shape && found < 0; ++u) {
+                    long long col = 0;
+                    for (int a = 0; a < 3; ++a) {
+                        const int i = (rc[a] + op.delta[u][a] + op.dims[a]) % op.dims[a];
+                        col = col * op.dims[a] + i;
+                    }
+                    if (col == op.exc_col[e]) found = u;
+                }
+                ok = found >= 0;
+                if (ok) c[(size_t)q * persist.shape + found] = T(op.exc_val[e]);
+                t = found;
+            }
+            list[q] = !ok;
+            any_list |= !ok;
+        }
+        const size_t wb = w.size() * sizeof(uint2), cb = c.size() * sizeof(T);
+        std::vector<unsigned char> h(wb + cb + list.size());
+        std::memcpy(h.data(), w.data(), wb);
+        std::memcpy(h.data() + wb, c.data(), cb);
+        std::memcpy(h.data() + wb + cb, list.data(), list.size());
+        rows.upload(h.data(), h.size(), s);
+        cuda_check(cudaStreamSynchronize(s), "upload stencil");
+        persist.word = reinterpret_cast<const uint2*>(rows.p);
+        persist.dense = reinterpret_cast<const T*>(rows.p + wb);
+        persist.csr = any_list ? rows.p + wb + cb : nullptr;
     }
 };
 
@@ -90,7 +149,22 @@ template <class T>
 struct DevAxis {
     DevBuf<int> p_c0, p_c1, r_f;
     DevBuf<T> p_w0, p_w1, r_w;
+    // The same factors as whole entries (one-kernel solve).
+    static void entries(const Axis1D& a, RestrictEntry<T>* re, ProlongEntry<T>* pe) {
+        for (int c = 0; c < a.nc; ++c)
+            for (int q = 0; q < 3; ++q) {
+                re[c].f[q] = std::max(0, a.r_f[3 * c + q]);
+                re[c].w[q] = a.r_f[3 * c + q] < 0 ? T(0) : T(a.r_w[3 * c + q]);
+            }
+        for (int f = 0; f < a.nf; ++f) {
+            pe[f].c[0] = std::max(0, a.p_c0[f]);
+            pe[f].c[1] = std::max(0, a.p_c1[f]);
+            pe[f].w[0] = a.p_c0[f] < 0 ? T(0) : T(a.p_w0[f]);
+            pe[f].w[1] = a.p_c1[f] < 0 ? T(0) : T(a.p_w1[f]);
+        }
+    }
     void upload(const Axis1D& a, cudaStream_t s, AxisDev<T>& view) {
+
         std::vector<T> w0(a.p_w0.begin(), a.p_w0.end()), w1(a.p_w1.begin(), a.p_w1.end()),
             rw(a.r_w.begin(), a.r_w.end());
         p_c0.upload(a.p_c0.data(), a.p_c0.size(), s);
@@ -215,19 +289,26 @@ void launch_tma_ns(TmapCache& cache, const StencilDev<T>& A, const T* x, const T
     k_level_op_tma<T, Mode, NS><<<blocks, kTmaThreads, S::smem(), s>>>(map, A, V, x, b, out, omega, st, stall);
 }
 
-// TMA-staged sweep of a level (k_level_op_tma); false when the level does
-// not qualify (small, not 3-D, or rows not a multiple of 16 bytes).
-template <class T, int Mode>
-bool launch_level_op_tma(TmapCache& cache, long long min_rows, const StencilDev<T>& A, const T* x, const T* b, T* out,
-                         T omega, const MGState* st, int* stall, cudaStream_t s) {
-    if (Mode == kSmoothFromZero || A.n < min_rows) return false;
+// Whether the TMA-staged sweep takes a level: not small, 3-D, rows a multiple
+// of 16 bytes long, one of the kernel's two stencil shapes.
+template <class T>
+bool tma_level(const StencilDev<T>& A, long long min_rows) {
+    if (A.n < min_rows) return false;
     if (!(A.n0 > 2 && A.n1 > 1 && A.n2 > 1)) return false;          // 3-D boxes only (2-D levels stay in L2)
     if ((A.n2 * (int)sizeof(T)) % 16 != 0) return false;             // tensor-map row pitch: 16-byte multiple
-    if ((reinterpret_cast<uintptr_t>(x) & 15) != 0) return false;
     if (A.ns != 7 && A.ns != 27) return false;                         // the kernel's two stencil shapes
     for (int t = 0; t < A.ns; ++t)
         if (A.di[t] != tma_tap_d(A.ns, t, 0) || A.dj[t] != tma_tap_d(A.ns, t, 1) || A.dk[t] != tma_tap_d(A.ns, t, 2))
             return false;
+    return true;
+}
+
+// TMA-staged sweep of a level (k_level_op_tma); false when the level does not qualify.
+template <class T, int Mode>
+bool launch_level_op_tma(TmapCache& cache, long long min_rows, const StencilDev<T>& A, const T* x, const T* b, T* out,
+                         T omega, const MGState* st, int* stall, cudaStream_t s) {
+    if (Mode == kSmoothFromZero || !tma_level(A, min_rows)) return false;
+    if ((reinterpret_cast<uintptr_t>(x) & 15) != 0) return false;
     if (A.ns == 7) launch_tma_ns<T, Mode, 7>(cache, A, x, b, out, omega, st, stall, s);
     else launch_tma_ns<T, Mode, 27>(cache, A, x, b, out, omega, st, stall, s);
     count_launch();
@@ -260,6 +341,83 @@ void launch_residual64(const StencilDev<double>& A, const double* x, const doubl
     count_launch();
 }
 
+// ------------------------------------------------- one-kernel solves --
+// Which levels one kernel takes, and how its blocks meet.  Solves on a B200,
+// one launch per step against one kernel: 64^2 FP64 3.3 -> 0.43 ms, 256^2
+// mixed 4.4 -> 0.63, 1025^2 mixed 6.0 -> 1.24, 33 x 41 x 29 FP64 4.3 -> 1.7,
+// 128^3 mixed 7.2 -> 2.3 (14 cycles), 256^3 mixed 17.0 -> 14.1 (coarse levels
+// only; 21.4 with all levels inside: its finest level streams from HBM, where
+// the TMA-staged sweep is twice as fast).
+constexpr long long kPersistRows = 1LL << 21;     // largest level worked inside the kernel
+// Up to here one cluster of 16 blocks, above one block per SM: a cluster
+// barrier and its loads take about 1 us a step against 2.6, but 16 SMs sweep
+// 65536 rows in 3.4 us, as long as 148 take for 512 x 512.
+constexpr long long kClusterRows = 100000;
+constexpr long long kTailBytes = 176 << 10;       // rows x taps x element size a tail level may have ...
+constexpr long long kTailBytesGrid = 256 << 10;   // ... and under a grid barrier, which costs more than a slow sweep
+constexpr size_t kTailSmem = 200 << 10;           // shared memory of the tail's vectors
+
+inline int device_sms() {
+    static int sms = 0;
+    if (!sms) {
+        int dev = 0;
+        cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
+        cuda_check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "cudaDeviceGetAttribute");
+    }
+    return sms;
+}
+
+// Blocks of the whole-GPU kernel when `beside` particles are still being
+// written (the fused step's second pass): a block takes its SM, so the pass
+// goes on with the others, and the best share is the one whose solve ends
+// with the pass.  Steps of 512 particles per row (1025^2 nodes): 9.15 ms with
+// every SM, 8.78 with a quarter, 9.38 with 20 blocks; of 32 per row (128^3):
+// 6.6 ms with every SM, 6.5 with two thirds, 8.3 with a quarter.
+inline int persist_blocks(long long beside, long long rows) {
+    const int sms = device_sms();
+    if (beside <= 0) return sms;
+    return std::max(1, beside >= 256 * rows ? sms / 4 : sms * 2 / 3);
+}
+
+template <class T, int SYNC>
+void launch_persist_sync(const PersistArgs<T>& a, size_t smem, long long beside, cudaStream_t s) {
+    static bool attr = false;
+    if (!attr) {
+        cuda_check(cudaFuncSetAttribute(k_mg_persist<T, SYNC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)kTailSmem),
+                   "cudaFuncSetAttribute");
+        if (SYNC == kSyncCluster)
+            cuda_check(cudaFuncSetAttribute(k_mg_persist<T, SYNC>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1),
+                       "cudaFuncSetAttribute");
+        attr = true;
+    }
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(SYNC == kSyncBlock ? 1 : (SYNC == kSyncCluster ? kClusterBlocks : persist_blocks(beside, (long long)a.lv[0].n)));
+    cfg.blockDim = dim3(kPersistThreads<T>);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    if (SYNC == kSyncCluster) {
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = kClusterBlocks;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    } else {
+        at.id = cudaLaunchAttributeCooperative;
+        at.val.cooperative = 1;
+    }
+    cfg.attrs = &at;
+    cfg.numAttrs = SYNC == kSyncBlock ? 0 : 1;
+    cuda_check(cudaLaunchKernelEx(&cfg, k_mg_persist<T, SYNC>, a), "multigrid kernel launch");
+    count_launch();
+}
+
+template <class T>
+void launch_persist(const PersistArgs<T>& a, int sync, size_t smem, long long beside, cudaStream_t s) {
+    if (sync == kSyncBlock) launch_persist_sync<T, kSyncBlock>(a, smem, beside, s);
+    else if (sync == kSyncCluster) launch_persist_sync<T, kSyncCluster>(a, smem, beside, s);
+    else launch_persist_sync<T, kSyncGrid>(a, smem, beside, s);
+}
+
 template <class T>
 struct Level {
     long long n = 0;
@@ -268,6 +426,28 @@ struct Level {
     DevBuf<T> bufA, bufB, b;   // x ping-pong pair and right-hand side
     XferDev<T> xfer{};         // to the next coarser level
     DevAxis<T> axes[3];
+    DevBuf<unsigned char> entries;   // RestrictEntry and ProlongEntry tables of the three axes, one buffer
+    const RestrictEntry<T>* rest[3] = {};
+    const ProlongEntry<T>* prol[3] = {};
+    void upload_entries(const std::array<Axis1D, 3>& ax, cudaStream_t s) {
+        size_t at[6], bytes = 0;
+        for (int a = 0; a < 3; ++a) {
+            at[a] = bytes;
+            bytes += sizeof(RestrictEntry<T>) * ax[a].nc;
+            at[3 + a] = bytes = (bytes + 31) / 32 * 32;
+            bytes = (bytes + sizeof(ProlongEntry<T>) * ax[a].nf + 31) / 32 * 32;
+        }
+        std::vector<unsigned char> h(bytes);
+        for (int a = 0; a < 3; ++a)
+            DevAxis<T>::entries(ax[a], reinterpret_cast<RestrictEntry<T>*>(h.data() + at[a]),
+                                reinterpret_cast<ProlongEntry<T>*>(h.data() + at[3 + a]));
+        entries.upload(h.data(), bytes, s);
+        cuda_check(cudaStreamSynchronize(s), "upload transfer");
+        for (int a = 0; a < 3; ++a) {
+            rest[a] = reinterpret_cast<const RestrictEntry<T>*>(entries.p + at[a]);
+            prol[a] = reinterpret_cast<const ProlongEntry<T>*>(entries.p + at[3 + a]);
+        }
+    }
 };
 
 }  // namespace mgdetail
@@ -287,9 +467,11 @@ struct SolverBase {
     int null_space = 0;                     // option `null_space 0|1` (read by set_matrix)
     bool ns_built = false;                  // the hierarchy was built for a singular operator
     int use_graph = 1;                      // option `graph 0|1`: replay the solve as one CUDA graph
+    int use_persist = 1;                    // option `persist 0|1`: the solve, or its coarse levels, as one kernel
     int use_tma = 1;                        // option `tma 0|1`: TMA-staged sweeps on large levels
-    long long tma_min_rows = kTmaMinRows;   // option `tma_min_rows`: smallest level (rows) swept that way
+    long long tma_min_rows = 0;             // option `tma_min_rows`: smallest level (rows) swept that way (0: rule)
     unsigned long long n_row = 0;
+    long long beside = 0;                   // particles being written meanwhile (solver_solve_async)
     bool ready = false;
     cudaStream_t own_stream = nullptr;
     // The solve's launch sequence depends only on the options, the operator,
@@ -330,6 +512,7 @@ struct SolverBase {
     }
     cudaStream_t aux_stream = nullptr;      // captures the body of a conditional loop
     unsigned long long loop_kernels = 0;    // kernels captured into loop bodies (counted on the device)
+    virtual bool one_kernel() const { return false; }   // the solve is a single kernel: no graph is captured
     virtual void build_device(cudaStream_t s) = 0;
     virtual void enqueue_solve(double* b, double* x, cudaStream_t s) = 0;
 };
@@ -345,7 +528,7 @@ struct Solver : SolverBase {
         tmaps.e.clear();
         a0.upload(host.a0, s);
         dinv0.upload(host.dinv[0].data(), host.dinv[0].size(), s);
-        partials.alloc(kNormBlocks);
+        partials.alloc(std::max(kNormBlocks, kNormVWarps));
         state.alloc(1);
         lv.clear();
         for (int l = 0; l <= host.L; ++l) {
@@ -360,6 +543,7 @@ struct Solver : SolverBase {
             L->b.alloc(L->n + 16);
             if (l < host.L) {
                 for (int a = 0; a < 3; ++a) L->axes[a].upload(host.xfer[l][a], s, L->xfer.ax[a]);
+                L->upload_entries(host.xfer[l], s);
                 const AxisDev<T>* ax = L->xfer.ax;
                 L->xfer.divc12 = make_fastdiv((unsigned)(ax[1].nc * ax[2].nc));
                 L->xfer.divc2 = make_fastdiv((unsigned)ax[2].nc);
@@ -380,13 +564,137 @@ struct Solver : SolverBase {
     TmapCache tmaps;   // tensor maps of the level vectors (rebuilt with the hierarchy)
     int tma_level_vectors() const override { return (int)tmaps.e.size(); }
 
+    // One-kernel plan: the first level the kernel takes (0: the whole solve;
+    // L + 1: none), its tail and its barrier.
+    struct Plan {
+        int first = 0, tail = 0, sync = kSyncGrid;
+        bool dense_all = false;
+        size_t smem = 0;
+    };
+    Plan persist_plan() const {
+        Plan P;
+        const int L = host.L;
+        P.first = L + 1;
+        // mixed solves with graph 0 launch every kernel (profiling); the FP64 backend has the same launches either way
+        if (!use_persist || (precision == 32 && !use_graph) || L + 1 > kPersistLevels || L < 1) return P;
+        int first = 0;
+        while (first < L && (lv[first]->n > kPersistRows || (use_tma && tma_level(lv[first]->op.view, tma_rows()))))
+            ++first;
+        if (first >= L) return P;
+        size_t elems = 3 * (size_t)lv[L]->n;
+        if (elems * sizeof(T) > kTailSmem) return P;
+        const bool grid = lv[first]->n > kClusterRows;
+        int tail = L;
+        while (tail > first) {
+            const Level<T>& V = *lv[tail - 1];
+            if (V.n * V.op.view.ns * (long long)sizeof(T) > (grid ? kTailBytesGrid : kTailBytes) ||
+                (elems + 3 * (size_t)V.n) * sizeof(T) > kTailSmem)
+                break;
+            elems += 3 * (size_t)V.n;
+            --tail;
+        }
+        P.first = first;
+        P.tail = tail;
+        P.dense_all = lv[L]->n > kDenseTailRows;
+        P.smem = tail < L ? elems * sizeof(T) : 0;
+        P.sync = tail == first ? kSyncBlock : (grid ? kSyncGrid : kSyncCluster);
+        return P;
+    }
+    // Smallest level of the TMA-staged sweep: the option, or by rule 2^20 rows
+    // in a problem that is too large for one kernel.  A smaller problem is
+    // worked whole by one (128^3 nodes, 14 mixed cycles: 2.3 ms against 3.8
+    // with the finest level's sweeps TMA-staged and launched).
+    long long tma_rows() const {
+        if (tma_min_rows > 0) return tma_min_rows;
+        const bool whole = use_persist && !(precision == 32 && !use_graph) && lv[0]->n <= kPersistRows;
+        return whole ? kPersistRows + 1 : kTmaMinRows;
+    }
+    PersistArgs<T> persist_args(const Plan& P, double* b, double* x) {
+        PersistArgs<T> a{};
+        const int L = host.L;
+        int at = 0;
+        for (int l = L; l >= 0; --l) {
+            PersistLevel<T>& q = a.lv[l];
+            q.A = lv[l]->op.persist;
+            q.X = lv[l]->xfer;
+            for (int d = 0; d < 3; ++d) {
+                q.rest[d] = lv[l]->rest[d];
+                q.prol[d] = lv[l]->prol[d];
+            }
+            q.dim = q.A.s.n2 > 1 ? 3 : (q.A.s.n1 > 1 ? 2 : 1);
+            q.x[0] = lv[l]->bufA.p;
+            q.x[1] = lv[l]->bufB.p;
+            q.b = lv[l]->b.p;
+            q.dinv = lv[l]->dinv.p;
+            q.n = (int)lv[l]->n;
+            if (l >= P.tail) {
+                q.smem = at;
+                at += 3 * q.n;
+            }
+        }
+        if (precision == 64) a.lv[0].x[0] = reinterpret_cast<T*>(x64.p);
+        a.a0 = a0.persist;
+        a.dinv0 = dinv0.p;
+        a.coarse_inv = coarse_inv.p;
+        a.b = b;
+        a.x = x;
+        a.add_idx = d_add_idx.p;
+        a.add_val = d_add_val.p;
+        a.rep_idx = d_rep_idx.p;
+        a.rep_val = d_rep_val.p;
+        a.n_add = (long long)add_idx.size();
+        a.n_rep = (long long)rep_idx.size();
+        a.partials = partials.p;
+        a.st = state.p;
+        a.counter = &state.p->arrivals;
+        a.tol = tol;
+        a.first = P.first;
+        a.tail = P.tail;
+        a.last = L;
+        a.dense_all = P.dense_all;
+        a.pre = pre_relax;
+        a.post = post_relax;
+        a.max_cycles = max_cycles;
+        a.interval = correction_interval;
+        a.null_space = ns_built;
+        return a;
+    }
+    bool one_kernel() const override { return ready_levels() && persist_plan().first == 0; }
+    bool ready_levels() const { return (int)lv.size() == host.L + 1; }
+
+    // The whole solve as one kernel.
+    void enqueue_persist(const Plan& P, double* b, double* x, cudaStream_t s) {
+        PersistArgs<T> a = persist_args(P, b, x);
+        a.mode = precision == 64 ? kPersistFp64 : kPersistMixed;
+        cuda_check(cudaMemsetAsync(&state.p->stall, 0, 2 * sizeof(int), s), "memset");   // stall, arrivals
+        launch_persist(a, P.sync, P.smem, beside, s);
+    }
+
+    // One V-cycle from level P.first (its right-hand side restricted, its
+    // iterate zero) as one kernel; returns the buffer of its result.
+    T* enqueue_persist_cycle(const Plan& P, bool gated, cudaStream_t s) {
+        PersistArgs<T> a = persist_args(P, nullptr, nullptr);
+        a.mode = kPersistCycle;
+        a.n_add = a.n_rep = 0;
+        a.null_space = 0;
+        a.max_cycles = 1;
+        a.gated = gated;
+        if (P.sync == kSyncGrid)
+            cuda_check(cudaMemsetAsync(&state.p->arrivals, 0, sizeof(unsigned), s), "memset");
+        launch_persist(a, P.sync, P.smem, beside, s);
+        if (P.tail == P.first) return lv[P.first]->bufA.p;
+        const int sweeps = (pre_relax >= 2 ? pre_relax - 2 : 0) + post_relax;
+        return sweeps % 2 ? lv[P.first]->bufB.p : lv[P.first]->bufA.p;
+    }
+
     // Enqueue `cycles` V(pre,post) cycles on level-0 (x0 in/out, b0 = scaled rhs).
     // `x_is_zero`: the level-0 iterate starts at zero (first sweep simplified).
     // Returns the buffer holding the final level-0 iterate.
     T* enqueue_vcycles(T* x0, T* other0, T* b0, int cycles, bool x_is_zero, cudaStream_t s, bool gated = true) {
         const MGState* st = gated ? state.p : nullptr;
         const T omega = T(2.0 / 3);
-        const int L = host.L;
+        const Plan P = persist_plan();
+        const int L = std::min(host.L, P.first);   // levels below are launched one kernel per step
         std::vector<T*> xcur(L + 1), xoth(L + 1), bl(L + 1);
         xcur[0] = x0;
         xoth[0] = other0;
@@ -404,7 +712,7 @@ struct Solver : SolverBase {
                 launch_level_op<T, kSmoothFromZero>(V.op.view, xcur[l], bl[l], xoth[l], omega, st, s);
                 zero[l] = false;
             } else {
-                launch_level_op<T, kSmooth>(V.op.view, xcur[l], bl[l], xoth[l], omega, st, s, tma_stall(), &tmaps, tma_min_rows);
+                launch_level_op<T, kSmooth>(V.op.view, xcur[l], bl[l], xoth[l], omega, st, s, tma_stall(), &tmaps, tma_rows());
             }
             std::swap(xcur[l], xoth[l]);
         };
@@ -417,13 +725,16 @@ struct Solver : SolverBase {
                     { k_restrict<T><<<grid_for(lv[l + 1]->n), kThreads, 0, s>>>(V.xfer, bl[l], bl[l + 1], xcur[l + 1],
                                                                              lv[l + 1]->dinv.p, st); count_launch(); }
                 } else {
-                    launch_level_op<T, kResidual>(V.op.view, xcur[l], bl[l], xoth[l], omega, st, s, tma_stall(), &tmaps, tma_min_rows);
+                    launch_level_op<T, kResidual>(V.op.view, xcur[l], bl[l], xoth[l], omega, st, s, tma_stall(), &tmaps, tma_rows());
                     { k_restrict<T><<<grid_for(lv[l + 1]->n), kThreads, 0, s>>>(V.xfer, xoth[l], bl[l + 1],
                                                                              xcur[l + 1], lv[l + 1]->dinv.p, st); count_launch(); }
                 }
                 zero[l + 1] = true;
             }
-            {
+            if (L < host.L) {
+                xcur[L] = enqueue_persist_cycle(P, gated, s);
+                zero[L] = false;
+            } else {
                 const int n = (int)lv[L]->n;
                 { k_dense_mv<T><<<grid_for((long long)n * 32), kThreads, 0, s>>>(coarse_inv.p, bl[L], xcur[L], n, st); count_launch(); }
                 zero[L] = false;
@@ -523,6 +834,10 @@ struct Solver : SolverBase {
         MGState* st = state.p;
         if (ns_built && !rep_idx.empty())
             throw std::invalid_argument("multigrid: null_space 1 with fixed (replaced) nodes");
+        if (const Plan P = persist_plan(); P.first == 0) {
+            enqueue_persist(P, b, x, s);
+            return;
+        }
         enqueue_sources(b, s);
         // singular operator: solve for the consistent part of b (the mean-zero
         // projection; b is the solve's scratch like PSuM's source vector)
@@ -624,6 +939,7 @@ void solver_set_options(SolverBase* s, const char* options) {
         else if (key == "periodic_J") s->periodic[1] = parse_int(iss, key) != 0;
         else if (key == "periodic_K") s->periodic[2] = parse_int(iss, key) != 0;
         else if (key == "graph") s->use_graph = parse_int(iss, key) != 0;
+        else if (key == "persist") s->use_persist = parse_int(iss, key) != 0;
         else if (key == "tma") s->use_tma = parse_int(iss, key) != 0;
         else if (key == "tma_min_rows") {
             long long v = 0;
@@ -730,7 +1046,7 @@ void solver_set_source(SolverBase* s, bool replace, unsigned long long n, const 
     upload_sources(s);
 }
 
-void solver_solve_async(SolverBase* s, double* b, double* x, cudaStream_t stream) {
+void solver_solve_async(SolverBase* s, double* b, double* x, cudaStream_t stream, long long beside) {
     if (!s->ready) throw Error(PSUM_ERR_NOT_READY, "solve called before set_matrix");
     if (!b || !x) throw std::invalid_argument("solve: null device pointer");
     for (auto i : s->rep_idx)
@@ -738,7 +1054,8 @@ void solver_solve_async(SolverBase* s, double* b, double* x, cudaStream_t stream
     for (auto i : s->add_idx)
         if (i >= s->n_row) throw std::invalid_argument("set_source_addback: index out of range");
     cudaStream_t st = stream ? stream : s->own_stream;
-    if (s->use_graph && capturable(st)) {
+    s->beside = beside;
+    if (s->use_graph && !s->one_kernel() && capturable(st)) {
         if (!(s->graph.exec && s->graph.b == b && s->graph.x == x && s->graph.version == s->version))
             capture_solve(s, b, x, st);
         cuda_check(cudaGraphLaunch(s->graph.exec, st), "cudaGraphLaunch");
@@ -786,7 +1103,7 @@ void ft_solve(psum_field_solver_handle h, double* b, double* x) {
     cuda_check(cudaStreamSynchronize(s->own_stream), "solve sync");
     MGState st = solver_read_state(s, s->own_stream);
     if (st.status == PSUM_ERR_DIVERGED) throw Error(PSUM_ERR_DIVERGED, "multigrid: residual diverged");
-    if (st.stall) throw Error(PSUM_ERR_INTERNAL, "multigrid: a TMA-staged sweep stopped waiting for its copies");
+    if (st.stall) throw Error(PSUM_ERR_INTERNAL, "multigrid: a kernel stopped waiting (copy or barrier)");
 }
 
 void ft_set_options(psum_field_solver_handle h, const char* o) { solver_set_options(solver_from_handle(h), o); }
@@ -861,7 +1178,7 @@ EXPORT int psum_mg_solve(psum_field_solver_handle h, double* b_dev, double* x_de
     if (rc != PSUM_OK) return rc;
     if (status == PSUM_ERR_NOT_CONVERGED) set_last_error("multigrid: tol not reached within max_cycles");
     if (status == PSUM_ERR_DIVERGED) set_last_error("multigrid: residual diverged");
-    if (status == PSUM_ERR_INTERNAL) set_last_error("multigrid: a TMA-staged sweep stopped waiting for its copies");
+    if (status == PSUM_ERR_INTERNAL) set_last_error("multigrid: a kernel stopped waiting (copy or barrier)");
     return status;
 }
 

@@ -21,7 +21,8 @@ void solver_set_matrix(SolverBase* s, unsigned long long n_row, unsigned long lo
                        const unsigned long long* rows, const unsigned long long* cols, const double* vals);
 void solver_set_source(SolverBase* s, bool replace, unsigned long long n, const unsigned long long* idx,
                        const double* v);
-void solver_solve_async(SolverBase* s, double* b, double* x, cudaStream_t stream);
+// beside: particles that the caller's kernels on another stream are still writing meanwhile
+void solver_solve_async(SolverBase* s, double* b, double* x, cudaStream_t stream, long long beside = 0);
 void solver_destroy(SolverBase* s);
 cudaStream_t solver_stream(SolverBase* s);
 

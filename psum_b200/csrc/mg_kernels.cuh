@@ -35,7 +35,8 @@ struct MGState {
     int status;             // psum_status of the solve
     int cycles_run;         // device-side counts of a solve looping in a graph
     int refinements_run;
-    int stall;              // a TMA-staged sweep gave up waiting for a copy (never expected)
+    int stall;              // a wait was given up: a copy of a TMA-staged sweep, or a grid barrier (never expected)
+    unsigned arrivals;      // grid barrier of the one-kernel solve, zeroed (with stall) before its launch
 };
 
 template <class T>
@@ -404,10 +405,9 @@ __global__ void __launch_bounds__(kTmaThreads, 4) k_level_op_tma(const __grid_co
     // every issued plane was waited on: nothing is in flight at exit
 }
 
-// b_c = dinv_c * (R r_f), x_c = 0 at coarse row c
+// (R r_f) at coarse row c
 template <class T, bool RO>
-__device__ __forceinline__ void restrict_row(const XferDev<T>& X, const T* __restrict__ rf, T* __restrict__ bc,
-                                             T* __restrict__ xc, const T* __restrict__ dinv_c, int c) {
+__device__ __forceinline__ T restrict_value(const XferDev<T>& X, const T* __restrict__ rf, int c) {
     const int nc1 = X.ax[1].nc, nc2 = X.ax[2].nc;
     const int nf1 = X.ax[1].nf, nf2 = X.ax[2].nf;
     const int ci = (int)fastdiv((unsigned)c, X.divc12);
@@ -434,7 +434,14 @@ __device__ __forceinline__ void restrict_row(const XferDev<T>& X, const T* __res
             }
         }
     }
-    bc[c] = s * __ldg(dinv_c + c);
+    return s;
+}
+
+// b_c = dinv_c * (R r_f), x_c = 0 at coarse row c
+template <class T, bool RO>
+__device__ __forceinline__ void restrict_row(const XferDev<T>& X, const T* __restrict__ rf, T* __restrict__ bc,
+                                             T* __restrict__ xc, const T* __restrict__ dinv_c, int c) {
+    bc[c] = restrict_value<T, RO>(X, rf, c) * __ldg(dinv_c + c);
     xc[c] = T(0);
 }
 
@@ -797,6 +804,7 @@ __global__ void k_check(const double* __restrict__ partials, int nparts, MGState
         st->cycles_run = 0;
         st->refinements_run = 0;
         st->stall = 0;
+        st->arrivals = 0;
         return;
     }
     if (phase == 1) {

@@ -3148,7 +3148,10 @@ EXPORT int psum_pic_step(psum_pic_ctx* ctx, psum_field_solver_handle solver, dou
             }
             {
                 PhaseTimer t(ctx, 1);
-                solver_solve_async(sv, rho_dev, phi_dev, ctx->prio);
+                long long writing = 0;   // particles of the pending second passes
+                if (ctx->pending)
+                    for (auto& sp : ctx->sp) writing += sp->n;
+                solver_solve_async(sv, rho_dev, phi_dev, ctx->prio, writing);
                 t.stop();
             }
         } catch (...) {
