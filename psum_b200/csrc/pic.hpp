@@ -31,6 +31,7 @@ struct Species {
     DevBuf<unsigned> starts[2];
     int starts_cur = 0;
     bool sorted = false;              // state sorted by cell and starts valid
+    bool arranged = false;            // sorted at least once since the load: nearly in cell order
     bool keys_stale = false;          // sorted mixed state whose keys follow from starts but are not written
     // fused sorted step: per (class, cell) counts then group offsets, block
     // table, new per-cell counts and scan scratch (per species, so that the
@@ -62,6 +63,8 @@ struct psum_pic_ctx {
     psum_b200::DevBuf<double> partials;
     psum_b200::DevBuf<long long> ipartials;
     psum_b200::SortScratch sort;
+    psum_b200::DevBuf<unsigned> bin_cnt, bin_off, bin_tot;   // psum_pic_bin: per-cell counts, offsets, scan totals
+    psum_b200::DevBuf<unsigned long long> valid;             // psum_pic_count
     psum_b200::DevBuf<int> far_flag;          // per species: a particle moved more than one cell on an axis
     // The second passes of a fused step run on `side` after the first passes
     // (event ev_pass1) and overlap what the caller enqueues next on the
