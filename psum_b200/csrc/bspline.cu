@@ -279,10 +279,11 @@ constexpr int kAggGroups = 4;
 // the bits are too.  off holds the lane's per-axis node offsets; the
 // leader's are the group's.
 constexpr int kTrChunk = 16;
+constexpr int kTrRuns = 4;   // runs of lanes with one stencil that the transposed deposit takes
 struct TrScratch {
     unsigned lo[kTrChunk][33];
     unsigned hi[kTrChunk][33];
-    int off[3][8];
+    int off[kTrRuns][3][6];
 };
 
 template <int N0, int N1, int N2, int NA, class Q>
@@ -293,7 +294,7 @@ __device__ __forceinline__ void deposit_one_group(const Q& q_at, bool ok, int le
 #pragma unroll
         for (int a = 0; a < 3; ++a)
 #pragma unroll
-            for (int j = 0; j < NA; ++j) t.off[a][j] = off[a][j];
+            for (int j = 0; j < NA; ++j) t.off[0][a][j] = off[a][j];
     }
 #pragma unroll
     for (int base = 0; base < NN; base += kTrChunk) {
@@ -320,7 +321,72 @@ __device__ __forceinline__ void deposit_one_group(const Q& q_at, bool ok, int le
         shi += __shfl_xor_sync(0xffffffffu, shi, 16);
         const unsigned long long sum = ((unsigned long long)shi << 27) + slo;
         if (h == 0 && node < NN && sum)
-            atomicAdd(acc + (t.off[0][node / (N1 * N2)] + t.off[1][(node / N2) % N1] + t.off[2][node % N2]), sum);
+            atomicAdd(acc + (t.off[0][0][node / (N1 * N2)] + t.off[0][1][(node / N2) % N1] + t.off[0][2][node % N2]), sum);
+        __syncwarp();
+    }
+}
+
+// First lanes of the runs of lanes with one key.
+template <class K>
+__device__ __forceinline__ unsigned run_heads(K key, int lane) {
+    const K prev = __shfl_up_sync(0xffffffffu, key, 1);
+    return __ballot_sync(0xffffffffu, lane == 0 || key != prev);
+}
+
+// A warp over several cells of a state stored cell by cell: `heads` marks the
+// first lane of every run of lanes with one stencil (at most kTrRuns).  The
+// same transpose; lane j (with lane j + 16 over the other half of the warp)
+// walks its 16 lanes and issues one atomic per node at the end of every run.
+// A 3-D cell of 16 particles gives two or three runs, for which the two warp
+// reductions per node and group cost more (97^3 nodes, order 2, 16 per cell:
+// 2.57 -> 1.02 ms).
+template <int N0, int N1, int N2, int NA, class Q>
+__device__ __forceinline__ void deposit_runs(const Q& q_at, bool ok, unsigned heads, const int (&off)[3][NA],
+                                             unsigned long long* __restrict__ acc, TrScratch& t, int lane) {
+    constexpr int NN = N0 * N1 * N2;
+    if ((heads >> lane) & 1u) {
+        const int run = __popc(heads & ((1u << lane) - 1u));
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+#pragma unroll
+            for (int j = 0; j < NA; ++j) t.off[run][a][j] = off[a][j];
+    }
+    const int j = lane & (kTrChunk - 1), h = lane >> 4;
+    const unsigned mine = (heads >> (h * 16)) & 0xffffu;                       // heads in this half
+    const int run0 = __popc(heads & ((2u << (h * 16)) - 1u)) - 1;              // run of the half's first lane
+#pragma unroll
+    for (int base = 0; base < NN; base += kTrChunk) {
+#pragma unroll
+        for (int c = 0; c < kTrChunk; ++c) {
+            const int node = base + c;
+            if (node < NN) {
+                const unsigned long long q = ok ? q_at(node / (N1 * N2), (node / N2) % N1, node % N2) : 0ULL;
+                t.lo[c][lane] = (unsigned)(q & 0x7ffffffULL);
+                t.hi[c][lane] = (unsigned)(q >> 27);
+            }
+        }
+        __syncwarp();
+        const int node = base + j;
+        if (node < NN) {
+            const int n0 = node / (N1 * N2), n1 = (node / N2) % N1, n2 = node % N2;
+            int run = run0;
+            unsigned slo = 0, shi = 0;
+            auto flush = [&] {
+                const unsigned long long sum = ((unsigned long long)shi << 27) + slo;
+                if (sum) atomicAdd(acc + (t.off[run][0][n0] + t.off[run][1][n1] + t.off[run][2][n2]), sum);
+                slo = shi = 0;
+            };
+#pragma unroll
+            for (int l = 0; l < 16; ++l) {
+                if (l > 0 && ((mine >> l) & 1u)) {
+                    flush();
+                    ++run;
+                }
+                slo += t.lo[j][h * 16 + l];
+                shi += t.hi[j][h * 16 + l];
+            }
+            flush();
+        }
         __syncwarp();
     }
 }
@@ -369,6 +435,8 @@ __global__ void __launch_bounds__(kBsThreads) k_bs_deposit(BsGrid g, long long n
     __shared__ TrScratch tr[kBsThreads / 32];
     if (__popc(leaders) == 1) {
         deposit_one_group<S, S1, S2, S>(q_at, ok, __ffs(leaders) - 1, off, acc, tr[threadIdx.x >> 5], lane);
+    } else if (const unsigned heads = run_heads(key, lane); __popc(heads) <= kTrRuns) {
+        deposit_runs<S, S1, S2, S>(q_at, ok, heads, off, acc, tr[threadIdx.x >> 5], lane);
     } else if (__popc(leaders) <= kAggGroups) {
 #pragma unroll
         for (int k0 = 0; k0 < S; ++k0)
@@ -477,6 +545,8 @@ __global__ void __launch_bounds__(kBsThreads) k_bs_deposit_near(BsGrid g, long l
     __shared__ TrScratch tr[kBsThreads / 32];
     if (__popc(leaders) == 1) {
         deposit_one_group<E, E1, E2, E>(q_at, ok, __ffs(leaders) - 1, off, acc, tr[threadIdx.x >> 5], lane);
+    } else if (const unsigned heads = run_heads(gkey, lane); __popc(heads) <= kTrRuns) {
+        deposit_runs<E, E1, E2, E>(q_at, ok, heads, off, acc, tr[threadIdx.x >> 5], lane);
     } else if (__popc(leaders) <= kAggGroups) {
 #pragma unroll
         for (int k0 = 0; k0 < E; ++k0)
