@@ -106,7 +106,9 @@ EXPORT int psum_mg_hierarchy_info(psum_field_solver_handle h, int* levels, unsig
                                   unsigned long long* exception_rows_level0);
 /* Level vectors the TMA-staged sweep kernel has read so far (one tensor map
  * each): 0 with option `tma 0`, before the first solve, or when no level
- * qualifies (3-D, at least 2^16 rows, rows a multiple of 16 bytes long). */
+ * qualifies (3-D, rows a multiple of 16 bytes long, at least `tma_min_rows`
+ * rows; by default 2^20 in problems of more than 2^21 rows, smaller ones
+ * being solved whole by one kernel). */
 EXPORT int psum_mg_tma_sweeps(psum_field_solver_handle h, int* level_vectors);
 EXPORT int psum_mg_destroy(psum_field_solver_handle h);
 

@@ -24,6 +24,7 @@
 #include <cmath>
 #include <cstring>
 #include <memory>
+#include <mutex>
 #include <sstream>
 #include <string>
 #include <vector>
@@ -379,6 +380,74 @@ inline int persist_blocks(long long beside, long long rows) {
     return std::max(1, beside >= 256 * rows ? sms / 4 : sms * 2 / 3);
 }
 
+// Whole-GPU solves of one device in turn.  Their blocks wait for one another
+// and take an SM each, so two of them (two handles on two streams, two
+// threads) must not be placed side by side by halves: each waits for the
+// event of the one before.  Streams that are being captured are left alone
+// (a graph's launch is ordered by `Turn` in solver_solve_async).
+class Turn {
+    struct Device {
+        std::mutex m;
+        cudaEvent_t last = nullptr;
+    };
+    Device* d = nullptr;
+    cudaStream_t s;
+
+public:
+    Turn(cudaStream_t stream, bool needed) : s(stream) {
+        if (!needed) return;
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        cuda_check(cudaStreamIsCapturing(s, &cs), "cudaStreamIsCapturing");
+        if (cs != cudaStreamCaptureStatusNone) return;
+        static Device devices[64];
+        int dev = 0;
+        cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
+        if (dev < 0 || dev >= 64) throw Error(PSUM_ERR_INTERNAL, "device ordinal out of range");
+        devices[dev].m.lock();
+        d = &devices[dev];
+        const cudaError_t e = d->last ? cudaStreamWaitEvent(s, d->last, 0)
+                                      : cudaEventCreateWithFlags(&d->last, cudaEventDisableTiming);
+        if (e != cudaSuccess) {
+            d->m.unlock();
+            d = nullptr;
+            cuda_check(e, "order of whole-GPU solves");
+        }
+    }
+    Turn(const Turn&) = delete;
+    Turn& operator=(const Turn&) = delete;
+    ~Turn() {
+        if (!d) return;
+        cudaEventRecord(d->last, s);
+        d->m.unlock();
+    }
+};
+
+// Whether the GPU places a cluster of 16 blocks of the kernel.
+template <class T>
+bool cluster_fits() {
+    static const bool fits = [] {
+        if (cudaFuncSetAttribute(k_mg_persist<T, kSyncCluster>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTailSmem) !=
+                cudaSuccess ||
+            cudaFuncSetAttribute(k_mg_persist<T, kSyncCluster>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+            return false;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(kClusterBlocks);
+        cfg.blockDim = dim3(kPersistThreads<T>);
+        cfg.dynamicSmemBytes = kTailSmem;
+        cudaLaunchAttribute at{};
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = kClusterBlocks;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        int n = 0;
+        const cudaError_t e = cudaOccupancyMaxActiveClusters(&n, k_mg_persist<T, kSyncCluster>, &cfg);
+        if (e != cudaSuccess) cudaGetLastError();
+        return e == cudaSuccess && n >= 1;
+    }();
+    return fits;
+}
+
 template <class T, int SYNC>
 void launch_persist_sync(const PersistArgs<T>& a, size_t smem, long long beside, cudaStream_t s) {
     static bool attr = false;
@@ -386,9 +455,6 @@ void launch_persist_sync(const PersistArgs<T>& a, size_t smem, long long beside,
         cuda_check(cudaFuncSetAttribute(k_mg_persist<T, SYNC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         (int)kTailSmem),
                    "cudaFuncSetAttribute");
-        if (SYNC == kSyncCluster)
-            cuda_check(cudaFuncSetAttribute(k_mg_persist<T, SYNC>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1),
-                       "cudaFuncSetAttribute");
         attr = true;
     }
     cudaLaunchConfig_t cfg{};
@@ -407,6 +473,7 @@ void launch_persist_sync(const PersistArgs<T>& a, size_t smem, long long beside,
     }
     cfg.attrs = &at;
     cfg.numAttrs = SYNC == kSyncBlock ? 0 : 1;
+    const Turn turn(s, SYNC == kSyncGrid);
     cuda_check(cudaLaunchKernelEx(&cfg, k_mg_persist<T, SYNC>, a), "multigrid kernel launch");
     count_launch();
 }
@@ -513,6 +580,7 @@ struct SolverBase {
     cudaStream_t aux_stream = nullptr;      // captures the body of a conditional loop
     unsigned long long loop_kernels = 0;    // kernels captured into loop bodies (counted on the device)
     virtual bool one_kernel() const { return false; }   // the solve is a single kernel: no graph is captured
+    virtual bool waits_on_gpu() const { return false; }   // holds a kernel whose blocks wait over the whole GPU
     virtual void build_device(cudaStream_t s) = 0;
     virtual void enqueue_solve(double* b, double* x, cudaStream_t s) = 0;
 };
@@ -583,7 +651,7 @@ struct Solver : SolverBase {
         if (first >= L) return P;
         size_t elems = 3 * (size_t)lv[L]->n;
         if (elems * sizeof(T) > kTailSmem) return P;
-        const bool grid = lv[first]->n > kClusterRows;
+        const bool grid = lv[first]->n > kClusterRows || !cluster_fits<T>();
         int tail = L;
         while (tail > first) {
             const Level<T>& V = *lv[tail - 1];
@@ -660,6 +728,10 @@ struct Solver : SolverBase {
         return a;
     }
     bool one_kernel() const override { return ready_levels() && persist_plan().first == 0; }
+    bool waits_on_gpu() const override {
+        const Plan P = persist_plan();
+        return P.first <= host.L && P.sync == kSyncGrid;
+    }
     bool ready_levels() const { return (int)lv.size() == host.L + 1; }
 
     // The whole solve as one kernel.
@@ -1058,6 +1130,7 @@ void solver_solve_async(SolverBase* s, double* b, double* x, cudaStream_t stream
     if (s->use_graph && !s->one_kernel() && capturable(st)) {
         if (!(s->graph.exec && s->graph.b == b && s->graph.x == x && s->graph.version == s->version))
             capture_solve(s, b, x, st);
+        const Turn turn(st, s->waits_on_gpu());
         cuda_check(cudaGraphLaunch(s->graph.exec, st), "cudaGraphLaunch");
         add_launches(s->graph.kernels);
         return;

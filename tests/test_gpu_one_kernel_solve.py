@@ -8,6 +8,8 @@ that fit one block, one cluster, the whole GPU, and ones whose finest levels
 stay launched; rows that wrap, rows with coefficients of their own, stencils
 of no usual shape; no, one and three smoothing sweeps; coarse systems solved
 by one block and by all."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -92,13 +94,40 @@ def test_mean_zero_gauge(kind, nodes):
 
 
 @pytest.mark.parametrize("kind", BACKENDS)
-def test_launched_finest_level(kind):
-    """A level that the TMA-staged sweep takes stays launched; the levels below it are one kernel per cycle."""
-    opts = ("I 48 J 48 K 48 depth 3 pre_relax 2 post_relax 1 max_cycles 6 correction_interval 2 tol 1e-9 "
-            "periodic_I 1 periodic_J 1 periodic_K 1 tma_min_rows 65536")
-    r, c, v, b, fixed = box((48, 48, 48), True)
+@pytest.mark.parametrize("nodes,min_rows", [((48, 48, 48), 1 << 16), ((128, 128, 64), 1 << 20)])
+def test_launched_finest_level(kind, nodes, min_rows):
+    """A level that the TMA-staged sweep takes stays launched; the levels below it are one kernel per cycle (of one
+    cluster, of one block per SM), captured into the solve's graph and its conditional loop."""
+    opts = (f"I {nodes[0]} J {nodes[1]} K {nodes[2]} depth 3 pre_relax 2 post_relax 1 max_cycles 6 correction_interval 2 "
+            f"tol 1e-9 periodic_I 1 periodic_J 1 periodic_K 1 tma_min_rows {min_rows}")
+    r, c, v, b, fixed = box(nodes, True)
     one, many = both(kind, opts, r, c, v, b, fixed=fixed)
     assert 1 < one[4] < many[4]
+
+
+@pytest.mark.parametrize("kind", BACKENDS)
+@pytest.mark.parametrize("nodes", [(64, 48), (96, 200), (400, 410)])
+def test_captured_by_the_caller(kind, nodes):
+    """A solve on a stream that the caller captures replays in the caller's graph with the bits of a direct one."""
+    opts = f"I {nodes[0]} J {nodes[1]} depth 4 pre_relax 2 post_relax 2 max_cycles 8 correction_interval 2 tol 1e-9"
+    r, c, v, b, fixed = box(nodes, False)
+    s = P.solver_backend(kind)
+    s.set_options(opts)
+    s.set_matrix(b.size, b.size, r.size, r, c, v)
+    bd, x, y = (torch.tensor(q, device="cuda") for q in (b, 0 * b, 0 * b))
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    s.solve_async(bd, x, stream)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=stream):
+        s.solve_async(bd, y, stream)
+    for _ in range(2):
+        y.zero_()
+        g.replay()
+        torch.cuda.synchronize()
+        assert (x == y).all()
+    g.reset()
 
 
 @pytest.mark.parametrize("kind", BACKENDS)
@@ -119,3 +148,38 @@ def test_unusual_stencils(kind):
         b = np.random.default_rng(3).normal(size=p.grid.n_nodes)
         both(kind, opts + " pre_relax 2 post_relax 2 max_cycles 6 correction_interval 2 tol 1e-8", r, c, v, b,
              fixed=p.replace_idx, value=0.5)
+
+
+def enqueue(s, stream, bs, xs):
+    for b, x in zip(bs, xs):
+        s.solve_async(b, x, stream)
+
+
+@pytest.mark.parametrize("nodes", [(400, 410), (96, 96)])
+def test_handles_on_two_streams_and_threads(nodes):
+    """Solves of two handles on two streams, enqueued by two threads without a wait between them, equal solves alone."""
+    r, c, v, b, fixed = box(nodes, False)
+    opts = f"I {nodes[0]} J {nodes[1]} depth 4 pre_relax 2 post_relax 2 max_cycles 12 correction_interval 2 tol 1e-9"
+    ref = solve(BACKENDS[0], opts, r, c, v, b)[0]
+    runs = []
+    for _ in range(2):
+        s = P.solver_backend(BACKENDS[0])
+        s.set_options(opts)
+        s.set_matrix(b.size, b.size, r.size, r, c, v)
+        st = torch.cuda.Stream()
+        with torch.cuda.stream(st):
+            runs.append((s, st, [torch.tensor(b, device="cuda") for _ in range(8)],
+                         [torch.tensor(np.random.default_rng(1).normal(size=b.size) * 0.1, device="cuda") for _ in range(8)]))
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=enqueue, args=run) for run in runs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    for s, _, _, xs in runs:
+        assert s.last_stats()["rel_residual"] <= 1e-9
+        for x in xs[1:]:
+            assert (x == xs[0]).all()
+    assert (runs[0][3][0] == runs[1][3][0]).all()
+    assert np.linalg.norm(runs[0][3][0].cpu().numpy() - ref) <= 1e-6 * np.linalg.norm(ref)
