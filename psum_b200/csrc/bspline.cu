@@ -155,8 +155,14 @@ __device__ __forceinline__ bool axis_support(const BsGrid& g, int a, double p, i
     return ok;
 }
 
+// Bound by the latency of its field loads (L1 and L2), so by the warps in
+// flight: four blocks per SM (64 registers) wherever they need no spills, two
+// for the 3-D orders 3 and 4.  67M positions stored cell by cell on 1024^2
+// nodes, gradient, two blocks against four: order 3 1.22 -> 1.13 ms, order 4
+// 2.01 -> 1.39; 97^3 nodes, order 2, 14M positions: 0.55 -> 0.37.  Five blocks
+// win another tenth at order 3 cell by cell and lose a fifth in random order.
 template <int D, int ORDER, bool GRAD>
-__global__ void __launch_bounds__(kBsThreads, 2) k_bs_gather(BsGrid g, long long n, const double* __restrict__ pos,
+__global__ void __launch_bounds__(kBsThreads, D == 3 && ORDER >= 3 ? 2 : 4) k_bs_gather(BsGrid g, long long n, const double* __restrict__ pos,
                                                           const double* __restrict__ field, double* __restrict__ out,
                                                           unsigned long long* __restrict__ skipped) {
     constexpr int S = ORDER + 1;
