@@ -4,6 +4,8 @@
 
 #include <cuda_runtime.h>
 
+#include <map>
+#include <mutex>
 #include <stdexcept>
 #include <string>
 
@@ -36,6 +38,25 @@ unsigned long long* device_launch_counter();
 inline void cuda_check(cudaError_t e, const char* what) {
     if (e != cudaSuccess) throw Error(PSUM_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
 }
+
+// What a device says once (a kernel's attributes set there, its resident
+// blocks, its SMs), kept per device ordinal: a process may use several.
+template <class V>
+class PerDevice {
+    std::mutex m;
+    std::map<int, V> known;
+
+public:
+    template <class F>
+    V get(F&& ask) {
+        int dev = 0;
+        cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
+        std::lock_guard<std::mutex> lk(m);
+        auto it = known.find(dev);
+        if (it == known.end()) it = known.emplace(dev, ask(dev)).first;
+        return it->second;
+    }
+};
 
 // Run `f`, translating exceptions into a status code and the thread's last
 // error message.

@@ -195,20 +195,21 @@ struct DevAxis {
 constexpr long long kTmaMinRows = 1LL << 20;
 
 // Blocks of a TMA-staged sweep that fit on the GPU at once (SMs x resident
-// blocks of the kernel), cached per kernel.
+// blocks of the kernel); the kernel's shared memory is allowed on the way.
 template <class T, int Mode, int NS>
 int tma_resident_blocks() {
-    static int blocks = 0;
-    if (!blocks) {
-        int dev = 0, sms = 0, per_sm = 0;
-        cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
+    static PerDevice<int> blocks;
+    return blocks.get([](int dev) {
+        int sms = 0, per_sm = 0;
+        cuda_check(cudaFuncSetAttribute(k_level_op_tma<T, Mode, NS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)TmaShape<T, NS>::smem()),
+                   "cudaFuncSetAttribute");
         cuda_check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "cudaDeviceGetAttribute");
         cuda_check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_level_op_tma<T, Mode, NS>, kTmaThreads,
                                                                  TmaShape<T, NS>::smem()),
                    "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
-        blocks = std::max(1, sms * std::max(1, per_sm));
-    }
-    return blocks;
+        return std::max(1, sms * std::max(1, per_sm));
+    });
 }
 
 // cuTensorMapEncodeTiled through the runtime's driver entry point (no link
@@ -268,13 +269,6 @@ template <class T, int Mode, int NS>
 void launch_tma_ns(TmapCache& cache, const StencilDev<T>& A, const T* x, const T* b, T* out, T omega,
                    const MGState* st, int* stall, cudaStream_t s) {
     using S = TmaShape<T, NS>;
-    static bool attr = false;
-    if (!attr) {
-        cuda_check(cudaFuncSetAttribute(k_level_op_tma<T, Mode, NS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)S::smem()),
-                   "cudaFuncSetAttribute");
-        attr = true;
-    }
     TmaTile V{};
     V.P = A.n0;
     V.R = A.n1;
@@ -359,13 +353,12 @@ constexpr long long kTailBytesGrid = 256 << 10;   // ... and under a grid barrie
 constexpr size_t kTailSmem = 200 << 10;           // shared memory of the tail's vectors
 
 inline int device_sms() {
-    static int sms = 0;
-    if (!sms) {
-        int dev = 0;
-        cuda_check(cudaGetDevice(&dev), "cudaGetDevice");
-        cuda_check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "cudaDeviceGetAttribute");
-    }
-    return sms;
+    static PerDevice<int> sms;
+    return sms.get([](int dev) {
+        int n = 0;
+        cuda_check(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev), "cudaDeviceGetAttribute");
+        return n;
+    });
 }
 
 // Blocks of the whole-GPU kernel when `beside` particles are still being
@@ -425,7 +418,8 @@ public:
 // Whether the GPU places a cluster of 16 blocks of the kernel.
 template <class T>
 bool cluster_fits() {
-    static const bool fits = [] {
+    static PerDevice<bool> fits;
+    return fits.get([](int) {
         if (cudaFuncSetAttribute(k_mg_persist<T, kSyncCluster>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTailSmem) !=
                 cudaSuccess ||
             cudaFuncSetAttribute(k_mg_persist<T, kSyncCluster>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
@@ -444,19 +438,18 @@ bool cluster_fits() {
         const cudaError_t e = cudaOccupancyMaxActiveClusters(&n, k_mg_persist<T, kSyncCluster>, &cfg);
         if (e != cudaSuccess) cudaGetLastError();
         return e == cudaSuccess && n >= 1;
-    }();
-    return fits;
+    });
 }
 
 template <class T, int SYNC>
 void launch_persist_sync(const PersistArgs<T>& a, size_t smem, long long beside, cudaStream_t s) {
-    static bool attr = false;
-    if (!attr) {
+    static PerDevice<bool> ready;
+    ready.get([](int) {
         cuda_check(cudaFuncSetAttribute(k_mg_persist<T, SYNC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         (int)kTailSmem),
                    "cudaFuncSetAttribute");
-        attr = true;
-    }
+        return true;
+    });
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(SYNC == kSyncBlock ? 1 : (SYNC == kSyncCluster ? kClusterBlocks : persist_blocks(beside, (long long)a.lv[0].n)));
     cfg.blockDim = dim3(kPersistThreads<T>);

@@ -2320,12 +2320,12 @@ template <int D, int P, int R>
 static void launch_pass_t(const ClsArgs& a, int pass, unsigned blocks, cudaStream_t s) {
     if (pass == 1) {
         constexpr size_t bytes = CellTileCap<D>::BYTES;
-        static bool attr = false;
-        if (!attr) {
+        static PerDevice<bool> ready;
+        ready.get([](int) {
             cuda_check(cudaFuncSetAttribute(k_cls_pass1<D, P, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes),
                        "cudaFuncSetAttribute");
-            attr = true;
-        }
+            return true;
+        });
         { k_cls_pass1<D, P, R><<<blocks, kPicThreads, bytes, s>>>(a); count_launch(); }
     } else {
         { k_cls_pass2<D, P, R><<<blocks, kPicThreads, 0, s>>>(a); count_launch(); }
