@@ -441,8 +441,30 @@ bool cluster_fits() {
     });
 }
 
+// Whether the device takes the whole-GPU kernel: launched cooperatively, one
+// block per SM.
+template <class T>
+bool whole_gpu_fits() {
+    static PerDevice<bool> fits;
+    return fits.get([](int dev) {
+        int coop = 0, per_sm = 0;
+        cuda_check(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev), "cudaDeviceGetAttribute");
+        if (!coop) return false;
+        if (cudaFuncSetAttribute(k_mg_persist<T, kSyncGrid>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTailSmem) !=
+                cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_mg_persist<T, kSyncGrid>, kPersistThreads<T>,
+                                                          kTailSmem) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        return per_sm >= 1;
+    });
+}
+
+// False where the device refuses the cooperative launch (a share of its SMs
+// only, whatever the attributes say).
 template <class T, int SYNC>
-void launch_persist_sync(const PersistArgs<T>& a, size_t smem, long long beside, cudaStream_t s) {
+bool launch_persist_sync(const PersistArgs<T>& a, size_t smem, long long beside, cudaStream_t s) {
     static PerDevice<bool> ready;
     ready.get([](int) {
         cuda_check(cudaFuncSetAttribute(k_mg_persist<T, SYNC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -467,15 +489,21 @@ void launch_persist_sync(const PersistArgs<T>& a, size_t smem, long long beside,
     cfg.attrs = &at;
     cfg.numAttrs = SYNC == kSyncBlock ? 0 : 1;
     const Turn turn(s, SYNC == kSyncGrid);
-    cuda_check(cudaLaunchKernelEx(&cfg, k_mg_persist<T, SYNC>, a), "multigrid kernel launch");
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, k_mg_persist<T, SYNC>, a);
+    if (SYNC == kSyncGrid && (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported)) {
+        cudaGetLastError();
+        return false;
+    }
+    cuda_check(e, "multigrid kernel launch");
     count_launch();
+    return true;
 }
 
 template <class T>
-void launch_persist(const PersistArgs<T>& a, int sync, size_t smem, long long beside, cudaStream_t s) {
-    if (sync == kSyncBlock) launch_persist_sync<T, kSyncBlock>(a, smem, beside, s);
-    else if (sync == kSyncCluster) launch_persist_sync<T, kSyncCluster>(a, smem, beside, s);
-    else launch_persist_sync<T, kSyncGrid>(a, smem, beside, s);
+bool launch_persist(const PersistArgs<T>& a, int sync, size_t smem, long long beside, cudaStream_t s) {
+    if (sync == kSyncBlock) return launch_persist_sync<T, kSyncBlock>(a, smem, beside, s);
+    if (sync == kSyncCluster) return launch_persist_sync<T, kSyncCluster>(a, smem, beside, s);
+    return launch_persist_sync<T, kSyncGrid>(a, smem, beside, s);
 }
 
 template <class T>
@@ -532,6 +560,7 @@ struct SolverBase {
     long long tma_min_rows = 0;             // option `tma_min_rows`: smallest level (rows) swept that way (0: rule)
     unsigned long long n_row = 0;
     long long beside = 0;                   // particles being written meanwhile (solver_solve_async)
+    bool whole_gpu = true;                  // false once the device has refused a whole-GPU kernel: launched kernels instead
     bool ready = false;
     cudaStream_t own_stream = nullptr;
     // The solve's launch sequence depends only on the options, the operator,
@@ -645,6 +674,7 @@ struct Solver : SolverBase {
         size_t elems = 3 * (size_t)lv[L]->n;
         if (elems * sizeof(T) > kTailSmem) return P;
         const bool grid = lv[first]->n > kClusterRows || !cluster_fits<T>();
+        const bool grid_ok = whole_gpu && whole_gpu_fits<T>();
         int tail = L;
         while (tail > first) {
             const Level<T>& V = *lv[tail - 1];
@@ -654,6 +684,7 @@ struct Solver : SolverBase {
             elems += 3 * (size_t)V.n;
             --tail;
         }
+        if (tail > first && grid && !grid_ok) return P;
         P.first = first;
         P.tail = tail;
         P.dense_all = lv[L]->n > kDenseTailRows;
@@ -727,16 +758,19 @@ struct Solver : SolverBase {
     }
     bool ready_levels() const { return (int)lv.size() == host.L + 1; }
 
-    // The whole solve as one kernel.
-    void enqueue_persist(const Plan& P, double* b, double* x, cudaStream_t s) {
+    // The whole solve as one kernel; false when the device refuses it.
+    bool enqueue_persist(const Plan& P, double* b, double* x, cudaStream_t s) {
         PersistArgs<T> a = persist_args(P, b, x);
         a.mode = precision == 64 ? kPersistFp64 : kPersistMixed;
         cuda_check(cudaMemsetAsync(&state.p->stall, 0, 2 * sizeof(int), s), "memset");   // stall, arrivals
-        launch_persist(a, P.sync, P.smem, beside, s);
+        const bool taken = launch_persist(a, P.sync, P.smem, beside, s);
+        if (!taken) whole_gpu = false;
+        return taken;
     }
 
     // One V-cycle from level P.first (its right-hand side restricted, its
-    // iterate zero) as one kernel; returns the buffer of its result.
+    // iterate zero) as one kernel; returns the buffer of its result, null when
+    // the device refuses the kernel.
     T* enqueue_persist_cycle(const Plan& P, bool gated, cudaStream_t s) {
         PersistArgs<T> a = persist_args(P, nullptr, nullptr);
         a.mode = kPersistCycle;
@@ -746,7 +780,10 @@ struct Solver : SolverBase {
         a.gated = gated;
         if (P.sync == kSyncGrid)
             cuda_check(cudaMemsetAsync(&state.p->arrivals, 0, sizeof(unsigned), s), "memset");
-        launch_persist(a, P.sync, P.smem, beside, s);
+        if (!launch_persist(a, P.sync, P.smem, beside, s)) {
+            whole_gpu = false;
+            return nullptr;
+        }
         if (P.tail == P.first) return lv[P.first]->bufA.p;
         const int sweeps = (pre_relax >= 2 ? pre_relax - 2 : 0) + post_relax;
         return sweeps % 2 ? lv[P.first]->bufB.p : lv[P.first]->bufA.p;
@@ -759,17 +796,17 @@ struct Solver : SolverBase {
         const MGState* st = gated ? state.p : nullptr;
         const T omega = T(2.0 / 3);
         const Plan P = persist_plan();
-        const int L = std::min(host.L, P.first);   // levels below are launched one kernel per step
-        std::vector<T*> xcur(L + 1), xoth(L + 1), bl(L + 1);
+        int L = std::min(host.L, P.first);   // levels below are launched one kernel per step
+        std::vector<T*> xcur(host.L + 1), xoth(host.L + 1), bl(host.L + 1);
         xcur[0] = x0;
         xoth[0] = other0;
         bl[0] = b0;
-        for (int l = 1; l <= L; ++l) {
+        for (int l = 1; l <= host.L; ++l) {
             xcur[l] = lv[l]->bufA.p;
             xoth[l] = lv[l]->bufB.p;
             bl[l] = lv[l]->b.p;
         }
-        std::vector<bool> zero(L + 1, false);
+        std::vector<bool> zero(host.L + 1, false);
         zero[0] = x_is_zero;
         auto smooth = [&](int l) {
             Level<T>& V = *lv[l];
@@ -781,8 +818,8 @@ struct Solver : SolverBase {
             }
             std::swap(xcur[l], xoth[l]);
         };
-        for (int c = 0; c < cycles; ++c) {
-            for (int l = 0; l < L; ++l) {
+        auto down = [&](int from) {
+            for (int l = from; l < L; ++l) {
                 for (int k = 0; k < pre_relax; ++k) smooth(l);
                 Level<T>& V = *lv[l];
                 if (zero[l]) {
@@ -796,8 +833,16 @@ struct Solver : SolverBase {
                 }
                 zero[l + 1] = true;
             }
-            if (L < host.L) {
-                xcur[L] = enqueue_persist_cycle(P, gated, s);
+        };
+        for (int c = 0; c < cycles; ++c) {
+            down(0);
+            T* coarse = L < host.L ? enqueue_persist_cycle(P, gated, s) : nullptr;
+            if (L < host.L && !coarse) {   // refused: these levels too are launched from here on
+                L = host.L;
+                down(P.first);
+            }
+            if (coarse) {
+                xcur[L] = coarse;
                 zero[L] = false;
             } else {
                 const int n = (int)lv[L]->n;
@@ -899,10 +944,7 @@ struct Solver : SolverBase {
         MGState* st = state.p;
         if (ns_built && !rep_idx.empty())
             throw std::invalid_argument("multigrid: null_space 1 with fixed (replaced) nodes");
-        if (const Plan P = persist_plan(); P.first == 0) {
-            enqueue_persist(P, b, x, s);
-            return;
-        }
+        if (const Plan P = persist_plan(); P.first == 0 && enqueue_persist(P, b, x, s)) return;
         enqueue_sources(b, s);
         // singular operator: solve for the consistent part of b (the mean-zero
         // projection; b is the solve's scratch like PSuM's source vector)
@@ -1121,8 +1163,23 @@ void solver_solve_async(SolverBase* s, double* b, double* x, cudaStream_t stream
     cudaStream_t st = stream ? stream : s->own_stream;
     s->beside = beside;
     if (s->use_graph && !s->one_kernel() && capturable(st)) {
-        if (!(s->graph.exec && s->graph.b == b && s->graph.x == x && s->graph.version == s->version))
-            capture_solve(s, b, x, st);
+        if (!(s->graph.exec && s->graph.b == b && s->graph.x == x && s->graph.version == s->version)) {
+            const bool whole = s->whole_gpu;
+            try {
+                capture_solve(s, b, x, st);
+            } catch (const Error&) {
+                // a graph (or the body of its loop) that may not hold the cooperative kernel: capture without it
+                if (!whole || (s->whole_gpu && !s->waits_on_gpu())) throw;
+                cudaGetLastError();
+                s->whole_gpu = false;
+                try {
+                    capture_solve(s, b, x, st);
+                } catch (...) {   // it failed for another reason
+                    s->whole_gpu = whole;
+                    throw;
+                }
+            }
+        }
         const Turn turn(st, s->waits_on_gpu());
         cuda_check(cudaGraphLaunch(s->graph.exec, st), "cudaGraphLaunch");
         add_launches(s->graph.kernels);

@@ -45,7 +45,7 @@ struct Graph {
 
 std::recursive_mutex mu;
 int device = 0;
-int sms[2] = {148, 100};
+int sms[8] = {148, 100, 148, 148, 148, 148, 148, 148};
 int refuse = 0;   // cooperative kernels: 1 refused at launch, 2 in a graph at its instantiation, 4 by the device's attribute
 cudaError_t last_error = cudaSuccess;
 std::map<const void*, std::string> names;

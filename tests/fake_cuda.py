@@ -111,6 +111,11 @@ class Solver:
     def set_options(self, options):
         self.check(self.lib.psum_mg_set_options(self.h, options.encode()))
 
+    def set_source(self, idx, values, replace=False):
+        idx, values = np.ascontiguousarray(idx, np.uint64), np.ascontiguousarray(values, np.float64)
+        f = self.lib.psum_mg_set_source_replace if replace else self.lib.psum_mg_set_source_addback
+        self.check(f(self.h, idx.size, idx.ctypes.data, values.ctypes.data))
+
     def check(self, code):
         assert code == 0, (code, self.lib.psum_last_error())
 

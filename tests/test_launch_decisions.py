@@ -42,3 +42,41 @@ def test_a_second_device_of_the_process(fake, kind, nodes, options, blocks):
         else:
             assert fake.kernels("k_level_op_tma")
         s.close()
+
+
+@pytest.mark.parametrize("kind", [M32, M64])
+@pytest.mark.parametrize("how", [1, 4])
+def test_whole_gpu_solve_refused(fake, kind, how):
+    """A device, or a share of one, that does not take the cooperative kernel solves with the launched kernels."""
+    if how == 4:
+        fake.lib.fake_device(2, 148)   # asked for once per device
+    fake.lib.fake_refuse_cooperative(how)
+    s = F.Solver(fake, kind, (400, 410))
+    s.set_source(np.array([7]), np.array([1.0]))
+    fake.lib.fake_clear_log()
+    st = fake.stream()
+    for _ in range(2):
+        s.check(s.solve_async(st))
+    assert not fake.kernels("k_mg_persist") and fake.kernels("k_level_op<")
+    assert len([q for q in fake.kernels("k_addback") if q.captured != 1]) == 2
+    s.close()
+
+
+@pytest.mark.parametrize("kind,options", [(M32, "tol 1e-9"), (M32, ""), (M64, "tol 1e-9")])
+@pytest.mark.parametrize("how", [1, 2])
+def test_whole_gpu_cycle_refused(fake, kind, options, how):
+    """The same for the kernel of a cycle's coarse levels, in the solve's graph (refused when it is instantiated) and
+    launched on a stream that takes no graph."""
+    fake.lib.fake_refuse_cooperative(how)
+    s = F.Solver(fake, kind, (64, 64, 272), "tma_min_rows 1000000 " + options)
+    s.set_source(np.array([7]), np.array([1.0]))
+    fake.lib.fake_clear_log()
+    st = fake.stream() if how == 2 else C.c_void_p(1)   # 1: the legacy default stream
+    for _ in range(2):
+        s.check(s.solve_async(st))
+    ran = [q for q in fake.log() if q.captured != 1]
+    assert not [q for q in ran if b"k_mg_persist" in q.name]
+    names = [q.name.split(b"<")[0].split(b"(")[0] for q in ran]
+    assert names.count(b"psum_b200::k_addback") == 2
+    assert sum(b"k_dense_mv" in n for n in names) > 0
+    s.close()
