@@ -376,8 +376,9 @@ inline int persist_blocks(long long beside, long long rows) {
 // Whole-GPU solves of one device in turn.  Their blocks wait for one another
 // and take an SM each, so two of them (two handles on two streams, two
 // threads) must not be placed side by side by halves: each waits for the
-// event of the one before.  Streams that are being captured are left alone
-// (a graph's launch is ordered by `Turn` in solver_solve_async).
+// event of the one before.  A solver's own graph is ordered where it is
+// launched (solver_solve_async); a graph of the caller's holds no such kernel
+// (SolverBase::callers_graph).
 class Turn {
     struct Device {
         std::mutex m;
@@ -560,6 +561,7 @@ struct SolverBase {
     long long tma_min_rows = 0;             // option `tma_min_rows`: smallest level (rows) swept that way (0: rule)
     unsigned long long n_row = 0;
     long long beside = 0;                   // particles being written meanwhile (solver_solve_async)
+    bool callers_graph = false;             // recorded into a graph that the caller replays when it likes
     bool whole_gpu = true;                  // false once the device has refused a whole-GPU kernel: launched kernels instead
     bool ready = false;
     cudaStream_t own_stream = nullptr;
@@ -674,7 +676,6 @@ struct Solver : SolverBase {
         size_t elems = 3 * (size_t)lv[L]->n;
         if (elems * sizeof(T) > kTailSmem) return P;
         const bool grid = lv[first]->n > kClusterRows || !cluster_fits<T>();
-        const bool grid_ok = whole_gpu && whole_gpu_fits<T>();
         int tail = L;
         while (tail > first) {
             const Level<T>& V = *lv[tail - 1];
@@ -684,7 +685,7 @@ struct Solver : SolverBase {
             elems += 3 * (size_t)V.n;
             --tail;
         }
-        if (tail > first && grid && !grid_ok) return P;
+        if (tail > first && grid && !grid_ok()) return P;
         P.first = first;
         P.tail = tail;
         P.dense_all = lv[L]->n > kDenseTailRows;
@@ -692,13 +693,14 @@ struct Solver : SolverBase {
         P.sync = tail == first ? kSyncBlock : (grid ? kSyncGrid : kSyncCluster);
         return P;
     }
+    bool grid_ok() const { return whole_gpu && !callers_graph && whole_gpu_fits<T>(); }
     // Smallest level of the TMA-staged sweep: the option, or by rule 2^20 rows
     // in a problem that is too large for one kernel.  A smaller problem is
     // worked whole by one (128^3 nodes, 14 mixed cycles: 2.3 ms against 3.8
     // with the finest level's sweeps TMA-staged and launched).
     long long tma_rows() const {
         if (tma_min_rows > 0) return tma_min_rows;
-        const bool whole = use_persist && !(precision == 32 && !use_graph) && lv[0]->n <= kPersistRows;
+        const bool whole = use_persist && !(precision == 32 && !use_graph) && lv[0]->n <= kPersistRows && grid_ok();
         return whole ? kPersistRows + 1 : kTmaMinRows;
     }
     PersistArgs<T> persist_args(const Plan& P, double* b, double* x) {
@@ -1104,11 +1106,14 @@ static void upload_sources(SolverBase* s) {
 // Graph capture needs a stream that is not the legacy/per-thread default
 // stream and is not already being captured by the caller (then the caller's
 // capture records the launches directly).
-static bool capturable(cudaStream_t st) {
-    if (st == nullptr || st == cudaStreamLegacy || st == cudaStreamPerThread) return false;
+static bool being_captured(cudaStream_t st) {
+    if (st == cudaStreamLegacy) return false;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     cuda_check(cudaStreamIsCapturing(st, &cs), "cudaStreamIsCapturing");
-    return cs == cudaStreamCaptureStatusNone;
+    return cs != cudaStreamCaptureStatusNone;
+}
+static bool capturable(cudaStream_t st) {
+    return st != nullptr && st != cudaStreamLegacy && st != cudaStreamPerThread && !being_captured(st);
 }
 
 static void capture_solve(SolverBase* s, double* b, double* x, cudaStream_t st) {
@@ -1162,6 +1167,7 @@ void solver_solve_async(SolverBase* s, double* b, double* x, cudaStream_t stream
         if (i >= s->n_row) throw std::invalid_argument("set_source_addback: index out of range");
     cudaStream_t st = stream ? stream : s->own_stream;
     s->beside = beside;
+    s->callers_graph = being_captured(st);
     if (s->use_graph && !s->one_kernel() && capturable(st)) {
         if (!(s->graph.exec && s->graph.b == b && s->graph.x == x && s->graph.version == s->version)) {
             const bool whole = s->whole_gpu;

@@ -80,3 +80,28 @@ def test_whole_gpu_cycle_refused(fake, kind, options, how):
     assert names.count(b"psum_b200::k_addback") == 2
     assert sum(b"k_dense_mv" in n for n in names) > 0
     s.close()
+
+
+@pytest.mark.parametrize("kind,nodes,options,one_kernel", [
+    (M32, (400, 410), "tol 1e-9", False), (M64, (400, 410), "", False), (M32, (64, 64, 272), "tol 1e-9 tma_min_rows 1000000", False),
+    (M64, (64, 64), "", True), (M32, (96, 96), "tol 1e-9", True)])
+def test_solve_captured_by_the_caller(fake, kind, nodes, options, one_kernel):
+    """The caller may replay its graphs beside one another and beside direct solves: nothing in them may wait for blocks
+    over the whole GPU.  One block, or one cluster, is placed whole and may."""
+    s = F.Solver(fake, kind, nodes, options)
+    st = fake.stream()
+    fake.lib.fake_clear_log()
+    s.check(s.solve_async(st))
+    assert any(q.cooperative for q in fake.log()) != one_kernel   # a direct solve takes the whole-GPU kernel
+    fake.lib.fake_clear_log()
+    assert fake.lib.cudaStreamBeginCapture(st, 0) == 0
+    s.check(s.solve_async(st))
+    g = C.c_void_p()
+    fake.lib.cudaStreamEndCapture(st, C.byref(g))
+    log = fake.log()
+    assert log and not any(q.cooperative for q in log)
+    assert (len(log) == 1) == one_kernel
+    fake.lib.fake_clear_log()
+    s.check(s.solve_async(st))   # and the next direct solve takes it again
+    assert any(q.cooperative for q in fake.log()) != one_kernel
+    s.close()
