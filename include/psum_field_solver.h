@@ -95,10 +95,14 @@ EXPORT int psum_mg_set_source_addback(psum_field_solver_handle h, unsigned long 
 EXPORT int psum_mg_solve(psum_field_solver_handle h, double* b_dev, double* x_dev);
 /* Asynchronous solve on `stream` (a cudaStream_t, NULL = the handle's own
  * stream).  No host synchronisation; convergence is decided on the device.
- * Read the outcome later with psum_mg_last_stats. */
+ * Read the outcome later with psum_mg_last_stats.  A solve whose kernel gave up
+ * a wait (bounded, never expected) is reported once as PSUM_ERR_INTERNAL, by
+ * the first of psum_mg_last_stats, psum_mg_solve, psum_mg_solve_async and
+ * psum_pic_step on the handle that comes after it. */
 EXPORT int psum_mg_solve_async(psum_field_solver_handle h, double* b_dev, double* x_dev, void* stream);
 /* Outcome of the last solve: V-cycles run, refinement steps run, final and
- * initial relative residual ||b - A x||_2 / ||b||_2 (FP64). Synchronises. */
+ * initial relative residual ||b - A x||_2 / ||b||_2 (FP64). Synchronises.
+ * PSUM_ERR_INTERNAL when a solve since the last report gave up a wait. */
 EXPORT int psum_mg_last_stats(psum_field_solver_handle h, int* cycles, int* refinements,
                               double* rel_residual, double* initial_rel_residual);
 /* Number of levels actually built and the coarsest level's size. */

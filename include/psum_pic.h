@@ -157,7 +157,9 @@ EXPORT int psum_pic_get_losses(psum_pic_ctx* ctx, unsigned long long* losses_hos
  * library's func_table (cuda_multigrid32f_gpu / cuda_multigrid64_gpu):
  *   rho = background + deposited charge  ->  solve A phi = rho  ->  push + deposit
  *   -> re-sort when due.  phi_dev is the initial guess and the output field;
- * rho_dev is scratch that receives the right-hand side.  Asynchronous. */
+ * rho_dev is scratch that receives the right-hand side.  Asynchronous.
+ * PSUM_ERR_INTERNAL, before anything is enqueued, when a solve of an earlier
+ * step gave up a wait; psum_mg_last_stats tells so after the last step. */
 EXPORT int psum_pic_step(psum_pic_ctx* ctx, psum_field_solver_handle solver, double background,
                          double* rho_dev, double* phi_dev, double dt, int pusher, const double* B);
 

@@ -222,6 +222,7 @@ class ElectrostaticRun:
                 nu = self._solve_t(mu)
                 for (sid, _, _), lx in zip(self.species, lam_x):
                     self.ctx.adjoint_deposit(sid, nu, lx)
+        self.solver.backend.last_stats()   # raises where a forward solve gave up a wait
         st = self.solver_t.last_stats()   # the last adjoint solve (synchronises)
         if not np.isfinite(st["rel_residual"]) or st["rel_residual"] > 1e-6:
             raise RuntimeError(f"adjoint solve did not converge: {st}")

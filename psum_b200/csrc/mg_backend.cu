@@ -267,7 +267,7 @@ struct TmapCache {
 // wave of resident blocks busy (each chunk re-reads two halo planes).
 template <class T, int Mode, int NS>
 void launch_tma_ns(TmapCache& cache, const StencilDev<T>& A, const T* x, const T* b, T* out, T omega,
-                   const MGState* st, int* stall, cudaStream_t s) {
+                   const MGState* st, Stall* stall, cudaStream_t s) {
     using S = TmaShape<T, NS>;
     TmaTile V{};
     V.P = A.n0;
@@ -301,7 +301,7 @@ bool tma_level(const StencilDev<T>& A, long long min_rows) {
 // TMA-staged sweep of a level (k_level_op_tma); false when the level does not qualify.
 template <class T, int Mode>
 bool launch_level_op_tma(TmapCache& cache, long long min_rows, const StencilDev<T>& A, const T* x, const T* b, T* out,
-                         T omega, const MGState* st, int* stall, cudaStream_t s) {
+                         T omega, const MGState* st, Stall* stall, cudaStream_t s) {
     if (Mode == kSmoothFromZero || !tma_level(A, min_rows)) return false;
     if ((reinterpret_cast<uintptr_t>(x) & 15) != 0) return false;
     if (A.ns == 7) launch_tma_ns<T, Mode, 7>(cache, A, x, b, out, omega, st, stall, s);
@@ -312,7 +312,7 @@ bool launch_level_op_tma(TmapCache& cache, long long min_rows, const StencilDev<
 
 template <class T, int Mode>
 void launch_level_op(const StencilDev<T>& A, const T* x, const T* b, T* out, T omega, const MGState* st,
-                     cudaStream_t s, int* stall = nullptr, TmapCache* cache = nullptr,
+                     cudaStream_t s, Stall* stall = nullptr, TmapCache* cache = nullptr,
                      long long tma_min_rows = kTmaMinRows) {
     if (stall && cache && launch_level_op_tma<T, Mode>(*cache, tma_min_rows, A, x, b, out, omega, st, stall, s)) return;
     const unsigned g = grid_for(A.n);
@@ -558,6 +558,7 @@ struct SolverBase {
     int use_graph = 1;                      // option `graph 0|1`: replay the solve as one CUDA graph
     int use_persist = 1;                    // option `persist 0|1`: the solve, or its coarse levels, as one kernel
     int use_tma = 1;                        // option `tma 0|1`: TMA-staged sweeps on large levels
+    int barrier_polls = kBarrierPolls;      // option `barrier_polls`: wait limit of a whole-GPU barrier
     long long tma_min_rows = 0;             // option `tma_min_rows`: smallest level (rows) swept that way (0: rule)
     unsigned long long n_row = 0;
     long long beside = 0;                   // particles being written meanwhile (solver_solve_async)
@@ -587,6 +588,7 @@ struct SolverBase {
     DevBuf<double> dinv0;
     DevBuf<double> partials;
     DevBuf<MGState> state;
+    int* stalled = nullptr;   // pinned, written by a kernel that gave up a wait (Stall::report)
     Hierarchy host;   // kept for introspection
     int levels = 0;
     unsigned long long coarse_rows = 0;
@@ -596,6 +598,7 @@ struct SolverBase {
         drop_graph();
         if (aux_stream) cudaStreamDestroy(aux_stream);
         if (own_stream) cudaStreamDestroy(own_stream);
+        if (stalled) cudaFreeHost(stalled);
     }
     void drop_graph() {
         if (graph.exec) cudaGraphExecDestroy(graph.exec);
@@ -621,7 +624,10 @@ struct Solver : SolverBase {
         a0.upload(host.a0, s);
         dinv0.upload(host.dinv[0].data(), host.dinv[0].size(), s);
         partials.alloc(std::max(kNormBlocks, kNormVWarps));
-        state.alloc(1);
+        MGState fresh{};
+        fresh.stall.report = stalled;
+        state.upload(&fresh, 1, s);
+        cuda_check(cudaStreamSynchronize(s), "build_device");
         lv.clear();
         for (int l = 0; l <= host.L; ++l) {
             auto L = std::make_unique<Level<T>>();
@@ -651,8 +657,8 @@ struct Solver : SolverBase {
         coarse_rows = (unsigned long long)lv.back()->n;
     }
 
-    // the stall word of the TMA-staged sweeps, or null when option `tma` is off
-    int* tma_stall() { return use_tma ? &state.p->stall : nullptr; }
+    // where the TMA-staged sweeps record a stall, or null when option `tma` is off
+    Stall* tma_stall() { return use_tma ? &state.p->stall : nullptr; }
     TmapCache tmaps;   // tensor maps of the level vectors (rebuilt with the hierarchy)
     int tma_level_vectors() const override { return (int)tmaps.e.size(); }
 
@@ -741,6 +747,7 @@ struct Solver : SolverBase {
         a.partials = partials.p;
         a.st = state.p;
         a.counter = &state.p->arrivals;
+        a.polls = barrier_polls;
         a.tol = tol;
         a.first = P.first;
         a.tail = P.tail;
@@ -764,7 +771,7 @@ struct Solver : SolverBase {
     bool enqueue_persist(const Plan& P, double* b, double* x, cudaStream_t s) {
         PersistArgs<T> a = persist_args(P, b, x);
         a.mode = precision == 64 ? kPersistFp64 : kPersistMixed;
-        cuda_check(cudaMemsetAsync(&state.p->stall, 0, 2 * sizeof(int), s), "memset");   // stall, arrivals
+        cuda_check(cudaMemsetAsync(&state.p->arrivals, 0, sizeof(unsigned), s), "memset");
         const bool taken = launch_persist(a, P.sync, P.smem, beside, s);
         if (!taken) whole_gpu = false;
         return taken;
@@ -1055,6 +1062,11 @@ void solver_set_options(SolverBase* s, const char* options) {
             if (!(iss >> v) || v < 1) throw std::invalid_argument("tma_min_rows must be positive");
             s->tma_min_rows = v;
         }
+        else if (key == "barrier_polls") {
+            int v = 0;
+            if (!(iss >> v) || v < 1) throw std::invalid_argument("barrier_polls must be positive");
+            s->barrier_polls = v;
+        }
         else if (key == "null_space") s->null_space = parse_int(iss, key) != 0;
         else if (key == "correction_interval") {
             int v = 0;
@@ -1087,6 +1099,12 @@ void solver_set_matrix(SolverBase* s, unsigned long long n_row, unsigned long lo
     // body of the conditional refinement loop, and the mapped launch counter
     if (!s->aux_stream) cuda_check(cudaStreamCreateWithFlags(&s->aux_stream, cudaStreamNonBlocking), "cudaStreamCreate");
     device_launch_counter();
+    if (!s->stalled) {
+        void* p = nullptr;
+        cuda_check(cudaHostAlloc(&p, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable), "cudaHostAlloc stall word");
+        s->stalled = static_cast<int*>(p);
+        *s->stalled = 0;
+    }
     s->version++;
     s->drop_graph();
     s->build_device(s->own_stream);
@@ -1158,8 +1176,15 @@ void solver_set_source(SolverBase* s, bool replace, unsigned long long n, const 
     upload_sources(s);
 }
 
+void solver_check_stall(SolverBase* s) {
+    if (s->stalled && __atomic_exchange_n(s->stalled, 0, __ATOMIC_ACQ_REL))
+        throw Error(PSUM_ERR_INTERNAL, "multigrid: a kernel of this or an earlier solve of the handle stopped waiting "
+                                       "(copy or barrier); its result is not a solution");
+}
+
 void solver_solve_async(SolverBase* s, double* b, double* x, cudaStream_t stream, long long beside) {
     if (!s->ready) throw Error(PSUM_ERR_NOT_READY, "solve called before set_matrix");
+    solver_check_stall(s);
     if (!b || !x) throw std::invalid_argument("solve: null device pointer");
     for (auto i : s->rep_idx)
         if (i >= s->n_row) throw std::invalid_argument("set_source_replace: index out of range");
@@ -1231,8 +1256,8 @@ void ft_solve(psum_field_solver_handle h, double* b, double* x) {
     solver_solve_async(s, b, x, s->own_stream);
     cuda_check(cudaStreamSynchronize(s->own_stream), "solve sync");
     MGState st = solver_read_state(s, s->own_stream);
+    solver_check_stall(s);
     if (st.status == PSUM_ERR_DIVERGED) throw Error(PSUM_ERR_DIVERGED, "multigrid: residual diverged");
-    if (st.stall) throw Error(PSUM_ERR_INTERNAL, "multigrid: a kernel stopped waiting (copy or barrier)");
 }
 
 void ft_set_options(psum_field_solver_handle h, const char* o) { solver_set_options(solver_from_handle(h), o); }
@@ -1302,12 +1327,12 @@ EXPORT int psum_mg_solve(psum_field_solver_handle h, double* b_dev, double* x_de
         SolverBase* s = solver_from_handle(h);
         solver_solve_async(s, b_dev, x_dev, s->own_stream);
         MGState st = solver_read_state(s, s->own_stream);
-        status = st.stall ? PSUM_ERR_INTERNAL : st.status;
+        solver_check_stall(s);
+        status = st.status;
     });
     if (rc != PSUM_OK) return rc;
     if (status == PSUM_ERR_NOT_CONVERGED) set_last_error("multigrid: tol not reached within max_cycles");
     if (status == PSUM_ERR_DIVERGED) set_last_error("multigrid: residual diverged");
-    if (status == PSUM_ERR_INTERNAL) set_last_error("multigrid: a kernel stopped waiting (copy or barrier)");
     return status;
 }
 
@@ -1325,6 +1350,7 @@ EXPORT int psum_mg_last_stats(psum_field_solver_handle h, int* cycles, int* refi
         if (!s->ready) throw Error(PSUM_ERR_NOT_READY, "no solve has run");
         cuda_check(cudaDeviceSynchronize(), "stats sync");
         MGState st = solver_read_state(s, s->own_stream);
+        solver_check_stall(s);
         const double bn = st.bnorm2 > 0 ? std::sqrt(st.bnorm2) : 1.0;
         if (cycles) *cycles = st.cycles;
         if (refinements) *refinements = st.refinements;

@@ -23,6 +23,8 @@ void solver_set_source(SolverBase* s, bool replace, unsigned long long n, const 
                        const double* v);
 // beside: particles that the caller's kernels on another stream are still writing meanwhile
 void solver_solve_async(SolverBase* s, double* b, double* x, cudaStream_t stream, long long beside = 0);
+// Throws PSUM_ERR_INTERNAL (once) when a solve of the handle gave up a wait.
+void solver_check_stall(SolverBase* s);
 void solver_destroy(SolverBase* s);
 cudaStream_t solver_stream(SolverBase* s);
 

@@ -25,6 +25,20 @@ namespace psum_b200 {
 constexpr int kMaxTaps = 27;
 constexpr int kThreads = 256;
 
+// A wait was given up (never expected): a copy of a TMA-staged sweep or a
+// barrier of the whole GPU.  `seen` ends the later waits of the same solve;
+// *report, a pinned word of the host's, stays set until the host has told the
+// caller, whichever solve was enqueued meanwhile.
+struct Stall {
+    int* report;
+    int seen;
+};
+__device__ __forceinline__ void record_stall(Stall* s) {
+    atomicExch(&s->seen, 1);
+    *(volatile int*)s->report = 1;
+    __threadfence_system();
+}
+
 struct MGState {
     double bnorm2;          // ||b||^2 after the source fix-ups
     double rnorm2_first;    // ||b - A x||^2 at the first check
@@ -35,8 +49,8 @@ struct MGState {
     int status;             // psum_status of the solve
     int cycles_run;         // device-side counts of a solve looping in a graph
     int refinements_run;
-    int stall;              // a wait was given up: a copy of a TMA-staged sweep, or a grid barrier (never expected)
-    unsigned arrivals;      // grid barrier of the one-kernel solve, zeroed (with stall) before its launch
+    unsigned arrivals;      // grid barrier of the one-kernel solve, zeroed before its launch
+    Stall stall;            // seen: zeroed by every solve
 };
 
 template <class T>
@@ -171,9 +185,9 @@ __global__ void __launch_bounds__(kThreads) k_level_op(StencilDev<T> A, const T*
 // the same CSR path, so the results are bit-identical to k_level_op.  b is
 // read one plane ahead into registers and out written directly (each once,
 // coalesced).  Every mbarrier wait
-// is bounded: after 2^16 suspended polls the block records a stall in
-// *stall, and once a stall is recorded later waits return at once, so a
-// wrong byte count cannot hang the GPU.  The tensor map covers only the
+// is bounded: after 2^16 suspended polls the block records a stall, and once
+// one is recorded the later waits of the solve return at once, so a wrong
+// byte count cannot hang the GPU.  The tensor map covers only the
 // solver's own level vector on this GPU; no multicast.
 struct TmaTile {
     int P, R, C;          // planes, rows, columns of the view (n0, n1, n2)
@@ -234,14 +248,14 @@ __device__ __forceinline__ bool mbar_try_wait(unsigned long long* bar, unsigned 
 }
 
 // Bounded wait for phase `parity` of bar: at most 2^16 suspended polls; on
-// expiry it records a stall in *stall and returns; once a stall is recorded
+// expiry it records a stall and returns; once a stall is recorded
 // (by this block or another) later waits return at once.
-__device__ __forceinline__ void mbar_wait_bounded(unsigned long long* bar, unsigned parity, int* stall) {
+__device__ __forceinline__ void mbar_wait_bounded(unsigned long long* bar, unsigned parity, Stall* stall) {
     if (mbar_try_wait(bar, parity)) return;
-    if (*(volatile int*)stall) return;
+    if (*(volatile int*)&stall->seen) return;
     for (int it = 0; it < (1 << 16); ++it)
         if (mbar_try_wait(bar, parity)) return;
-    atomicExch(stall, 1);
+    record_stall(stall);
 }
 
 // One tiled TMA load of the box at (x, y, z) of the tensor map into shared
@@ -258,7 +272,7 @@ template <class T, int Mode, int NS>
 __global__ void __launch_bounds__(kTmaThreads, 4) k_level_op_tma(const __grid_constant__ CUtensorMap xmap, StencilDev<T> A,
                                                               TmaTile V, const T* __restrict__ x,
                                                               const T* __restrict__ b, T* __restrict__ out, T omega,
-                                                              const MGState* __restrict__ st, int* stall) {
+                                                              const MGState* __restrict__ st, Stall* stall) {
     using S = TmaShape<T, NS>;
     constexpr int TC = S::TC, TR = S::TR, KA = S::KA, W = S::W, H = S::H;
     constexpr int NSL = S::SLOTS;
@@ -803,8 +817,8 @@ __global__ void k_check(const double* __restrict__ partials, int nparts, MGState
         st->status = 0;
         st->cycles_run = 0;
         st->refinements_run = 0;
-        st->stall = 0;
         st->arrivals = 0;
+        st->stall.seen = 0;
         return;
     }
     if (phase == 1) {

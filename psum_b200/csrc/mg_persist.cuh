@@ -25,9 +25,8 @@
 // residuals are those of the launched kernels bit for bit.
 //
 // Waits: a cluster barrier cannot spin; a grid barrier polls a counter at
-// most kBarrierPolls times, then records a stall in the solver's state word
-// (the solve returns PSUM_ERR_INTERNAL) and no later barrier of the block
-// waits.
+// most `polls` times, then records a stall and no later barrier of the block
+// waits.  The host reports a stall as PSUM_ERR_INTERNAL.
 #pragma once
 
 #include "mg_kernels.cuh"
@@ -42,7 +41,7 @@ constexpr int kPersistLevels = 12;
 constexpr int kClusterBlocks = 16;
 constexpr int kNormVBlocks = 444;           // the fixed grid of the norms: 444 blocks of 256 rows per stride
 constexpr int kNormVWarps = kNormVBlocks * 8;
-constexpr int kBarrierPolls = 1 << 22;
+constexpr int kBarrierPolls = 1 << 22;      // about 4 s
 constexpr int kDenseTailRows = 128;         // coarse systems up to this size are solved by the tail's block
 
 enum PersistSync { kSyncBlock = 0, kSyncCluster = 1, kSyncGrid = 2 };
@@ -102,6 +101,7 @@ struct PersistArgs {
     double* partials;             // kNormVWarps warp sums
     MGState* st;
     unsigned* counter;            // grid barrier
+    int polls;                    // its wait limit
     double tol;
     int mode;
     int first, tail, last;        // first level of this kernel, first tail level, coarsest level
@@ -115,7 +115,8 @@ struct PersistArgs {
 template <int SYNC>
 struct Barrier {
     unsigned* counter;
-    int* stall;
+    Stall* stall;
+    int polls;
     unsigned target = 0;
     bool broken = false;
 
@@ -135,9 +136,9 @@ struct Barrier {
                     for (;;) {
                         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(counter) : "memory");
                         if ((int)(v - target) >= 0) break;
-                        if (++it >= kBarrierPolls) {
+                        if (++it >= polls) {
                             broken = true;
-                            atomicExch(stall, 1);
+                            record_stall(stall);
                             break;
                         }
                     }
@@ -724,8 +725,8 @@ __global__ void __launch_bounds__(kPersistThreads<T>, 1) k_mg_persist(const __gr
     extern __shared__ __align__(16) unsigned char persist_smem[];
     __shared__ __align__(16) unsigned char level_smem[sizeof(PersistLevel<T>) * kPersistLevels];
     if (p.mode == kPersistCycle && p.gated && p.st->done) return;
-    Barrier<SYNC> sync{p.counter, &p.st->stall};
-    Barrier<kSyncBlock> bsync{nullptr, nullptr};
+    Barrier<SYNC> sync{p.counter, &p.st->stall, p.polls};
+    Barrier<kSyncBlock> bsync{nullptr, nullptr, 0};
     const int tid = blockIdx.x * NT + threadIdx.x, nthr = gridDim.x * NT;
     const int warp = tid >> 5, nwarps = nthr >> 5;
     const int n = (int)p.a0.s.n;

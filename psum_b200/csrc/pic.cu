@@ -3280,6 +3280,7 @@ EXPORT int psum_pic_step(psum_pic_ctx* ctx, psum_field_solver_handle solver, dou
             for (int si = 0; si < (int)ctx->sp.size() && si < 8; ++si) far |= ctx->far_host[si] != 0;
             if (far) finish_cls_step(ctx);
         }
+        solver_check_stall(sv);   // the last step's solve, where its first passes were waited for above
         cudaStream_t user = ctx->stream;
         if (ctx->diag) {
             if (ctx->sp.size() > 8) throw std::invalid_argument("step diagnostics: more than 8 species");

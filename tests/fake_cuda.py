@@ -131,3 +131,25 @@ class Solver:
 
     def close(self):
         self.lib.psum_mg_destroy(self.h)
+
+
+def step_context(fake, cells, per_cell=4, options="sort_interval 1"):
+    """A particle context with one species; returns a function that runs one step with a solver, and one to close it."""
+    lib, dim = fake.lib, len(cells)
+    g = _lib.GridDesc()
+    g.dim = dim
+    for a in range(3):
+        g.cells[a] = cells[a] if a < dim else 1
+        g.lower[a], g.upper[a], g.periodic[a] = 0.0, float(g.cells[a]), 0
+    ctx = C.c_void_p()
+    assert lib.psum_pic_create(C.byref(g), 0, C.byref(ctx)) == 0
+    assert lib.psum_pic_set_options(ctx, options.encode()) == 0
+    n, sid = per_cell * int(np.prod(cells)), C.c_int()
+    assert lib.psum_pic_add_species(ctx, C.byref(_lib.SpeciesDesc(1.0, 1.0, 1.0)), n, C.byref(sid)) == 0
+    pos, vel = np.full((dim, n), 0.5), np.zeros((3, n))
+    assert lib.psum_pic_load(ctx, sid.value, n, pos.ctypes.data, vel.ctypes.data) == 0
+    assert lib.psum_pic_sort(ctx) == 0 and lib.psum_pic_deposit(ctx) == 0
+
+    def step(solver):
+        return lib.psum_pic_step(ctx, solver.h, 0.0, solver.b.ctypes.data, solver.x.ctypes.data, 0.1, 0, (C.c_double * 3)())
+    return step, lambda: lib.psum_pic_destroy(ctx)
