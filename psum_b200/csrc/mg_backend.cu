@@ -789,7 +789,8 @@ struct Solver : SolverBase {
         a.gated = gated;
         if (P.sync == kSyncGrid)
             cuda_check(cudaMemsetAsync(&state.p->arrivals, 0, sizeof(unsigned), s), "memset");
-        if (!launch_persist(a, P.sync, P.smem, beside, s)) {
+        // on every SM: the graph that holds it is replayed whatever runs beside it
+        if (!launch_persist(a, P.sync, P.smem, 0, s)) {
             whole_gpu = false;
             return nullptr;
         }

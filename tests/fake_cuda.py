@@ -133,7 +133,7 @@ class Solver:
         self.lib.psum_mg_destroy(self.h)
 
 
-def step_context(fake, cells, per_cell=4, options="sort_interval 1"):
+def step_context(fake, cells, n=1000, options="sort_interval 1"):
     """A particle context with one species; returns a function that runs one step with a solver, and one to close it."""
     lib, dim = fake.lib, len(cells)
     g = _lib.GridDesc()
@@ -144,7 +144,7 @@ def step_context(fake, cells, per_cell=4, options="sort_interval 1"):
     ctx = C.c_void_p()
     assert lib.psum_pic_create(C.byref(g), 0, C.byref(ctx)) == 0
     assert lib.psum_pic_set_options(ctx, options.encode()) == 0
-    n, sid = per_cell * int(np.prod(cells)), C.c_int()
+    sid = C.c_int()
     assert lib.psum_pic_add_species(ctx, C.byref(_lib.SpeciesDesc(1.0, 1.0, 1.0)), n, C.byref(sid)) == 0
     pos, vel = np.full((dim, n), 0.5), np.zeros((3, n))
     assert lib.psum_pic_load(ctx, sid.value, n, pos.ctypes.data, vel.ctypes.data) == 0

@@ -122,3 +122,29 @@ def test_a_stall_is_told_by_the_next_call(fake):
         assert call() == 0
     close()
     s.close()
+
+
+def test_graph_of_a_solve_is_the_same_beside_a_pending_pass(fake):
+    """A graph captured while a fused step's second pass is pending is replayed by solves that run alone: its kernels
+    take every SM whatever was pending at the capture.  A whole solve as one kernel is launched each time and leaves
+    SMs to the pass."""
+    nodes = (64, 64, 272)
+    s = F.Solver(fake, M32, nodes, "tma_min_rows 1000000")
+    step, close = F.step_context(fake, tuple(k - 1 for k in nodes), n=1000)
+    assert step(s) == 0 and step(s) == 0
+    s.set_options("K 272 max_cycles 2")   # the graph is captured again, beside the pending pass
+    fake.lib.fake_clear_log()
+    assert step(s) == 0
+    assert fake.kernels("k_cls_pass2")    # there is one
+    s.check(s.solve_async(fake.stream()))
+    assert {q.grid for q in fake.kernels("k_mg_persist") if q.captured != 1} == {148}
+    close()
+    s.close()
+    one = F.Solver(fake, M32, (401, 401))
+    step, close = F.step_context(fake, (400, 400), n=1000)
+    fake.lib.fake_clear_log()
+    assert step(one) == 0 and step(one) == 0
+    a, b = (q.grid for q in fake.kernels("k_mg_persist"))
+    assert a == 148 > b
+    close()
+    one.close()
