@@ -87,7 +87,6 @@ struct DevStencil {
         view.exc_ptr = exc_ptr.p;
         view.exc_col = exc_col.p;
         view.exc_val = exc_val.p;
-        upload_persist(op, s);
     }
 
     // The stencil's shape, and every exception row as coefficients on the
@@ -609,6 +608,7 @@ struct SolverBase {
     virtual bool one_kernel() const { return false; }   // the solve is a single kernel: no graph is captured
     virtual bool waits_on_gpu() const { return false; }   // holds a kernel whose blocks wait over the whole GPU
     virtual void build_device(cudaStream_t s) = 0;
+    virtual void build_persist(cudaStream_t s) = 0;   // tables of the one-kernel solve, unless they are there
     virtual void enqueue_solve(double* b, double* x, cudaStream_t s) = 0;
 };
 
@@ -622,6 +622,7 @@ struct Solver : SolverBase {
     void build_device(cudaStream_t s) override {
         tmaps.e.clear();
         a0.upload(host.a0, s);
+        persist_tables = false;
         dinv0.upload(host.dinv[0].data(), host.dinv[0].size(), s);
         partials.alloc(std::max(kNormBlocks, kNormVWarps));
         MGState fresh{};
@@ -641,7 +642,6 @@ struct Solver : SolverBase {
             L->b.alloc(L->n + 16);
             if (l < host.L) {
                 for (int a = 0; a < 3; ++a) L->axes[a].upload(host.xfer[l][a], s, L->xfer.ax[a]);
-                L->upload_entries(host.xfer[l], s);
                 const AxisDev<T>* ax = L->xfer.ax;
                 L->xfer.divc12 = make_fastdiv((unsigned)(ax[1].nc * ax[2].nc));
                 L->xfer.divc2 = make_fastdiv((unsigned)ax[2].nc);
@@ -652,9 +652,25 @@ struct Solver : SolverBase {
         }
         coarse_inv.upload(host.coarse_inv.data(), host.coarse_inv.size(), s);
         if (precision == 64) x64.alloc(n_row + 16);
+        if (use_persist) build_persist(s);
         cuda_check(cudaStreamSynchronize(s), "build_device");
         levels = host.L + 1;
         coarse_rows = (unsigned long long)lv.back()->n;
+    }
+
+    // The operators and transfers as the one-kernel solve reads them, for the
+    // levels that it can work (with varying coefficients many rows
+    // are exception rows: 40 to 216 bytes more each).
+    bool persist_tables = false;
+    void build_persist(cudaStream_t s) override {
+        if (persist_tables || host.L < 1 || host.L + 1 > kPersistLevels) return;
+        for (int l = 0; l < host.L; ++l) {
+            if (lv[l]->n > kPersistRows) continue;
+            lv[l]->op.upload_persist(host.ahat[l], s);
+            lv[l]->upload_entries(host.xfer[l], s);
+        }
+        if (lv[0]->n <= kPersistRows) a0.upload_persist(host.a0, s);
+        persist_tables = true;
     }
 
     // where the TMA-staged sweeps record a stall, or null when option `tma` is off
@@ -674,7 +690,7 @@ struct Solver : SolverBase {
         const int L = host.L;
         P.first = L + 1;
         // mixed solves with graph 0 launch every kernel (profiling); the FP64 backend has the same launches either way
-        if (!use_persist || (precision == 32 && !use_graph) || L + 1 > kPersistLevels || L < 1) return P;
+        if (!use_persist || !persist_tables || (precision == 32 && !use_graph)) return P;
         int first = 0;
         while (first < L && (lv[first]->n > kPersistRows || (use_tma && tma_level(lv[first]->op.view, tma_rows()))))
             ++first;
@@ -706,7 +722,7 @@ struct Solver : SolverBase {
     // with the finest level's sweeps TMA-staged and launched).
     long long tma_rows() const {
         if (tma_min_rows > 0) return tma_min_rows;
-        const bool whole = use_persist && !(precision == 32 && !use_graph) && lv[0]->n <= kPersistRows && grid_ok();
+        const bool whole = use_persist && persist_tables && !(precision == 32 && !use_graph) && lv[0]->n <= kPersistRows && grid_ok();
         return whole ? kPersistRows + 1 : kTmaMinRows;
     }
     PersistArgs<T> persist_args(const Plan& P, double* b, double* x) {
@@ -1086,6 +1102,7 @@ void solver_set_options(SolverBase* s, const char* options) {
     if (s->pre_relax < 0 || s->post_relax < 0 || s->max_cycles < 0 || s->depth < 1)
         throw std::invalid_argument("set_options: negative relax/cycle counts or depth < 1");
     s->version++;
+    if (s->ready && s->use_persist) s->build_persist(s->own_stream);
 }
 
 void solver_set_matrix(SolverBase* s, unsigned long long n_row, unsigned long long n_col, unsigned long long nnz,

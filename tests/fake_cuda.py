@@ -91,8 +91,7 @@ def poisson(nodes, eps=None):
     cols.append(idx[inner])
     vals.append(diag[inner])
     r, c, v = (np.concatenate(q) for q in (rows, cols, vals))
-    o = np.lexsort((c, r))
-    return r[o].astype(np.uint64), c[o].astype(np.uint64), np.ascontiguousarray(v[o])
+    return r.astype(np.uint64), c.astype(np.uint64), v
 
 
 class Solver:

@@ -148,3 +148,34 @@ def test_graph_of_a_solve_is_the_same_beside_a_pending_pass(fake):
     assert a == 148 > b
     close()
     one.close()
+
+
+def test_tables_only_where_a_kernel_reads_them(fake):
+    """The one-kernel solve's own copies of the exception rows (with varying coefficients: many) are made
+    for the levels that it can work, and not with `persist 0`."""
+    def bytes_of(nodes, options):
+        before = fake.lib.fake_device_bytes()
+        eps = 1.0 + np.random.default_rng(2).random(nodes[0])   # per row of nodes; the uniform half gives the stencil
+        eps[:nodes[0] // 2] = 1.0
+        s = F.Solver(fake, M64, nodes, options, eps=np.broadcast_to(eps[:, None], nodes))
+        return s, fake.lib.fake_device_bytes() - before
+
+    nodes = (160, 160)
+    s1, with_ = bytes_of(nodes, "persist 1")
+    s0, without = bytes_of(nodes, "persist 0")
+    assert with_ - without > 160 * 160 // 2 * 5 * 8       # the fine operator's exception rows alone
+    before = fake.lib.fake_device_bytes()
+    s0.set_options("persist 1")                           # asked for later: made then
+    assert fake.lib.fake_device_bytes() - before == with_ - without
+    fake.lib.fake_clear_log()
+    s0.check(s0.solve_async(fake.stream()))
+    assert len(fake.log()) == 1
+    s0.close()
+    s1.close()
+    nodes = (1049, 2000)                                  # 1000 rows above the largest level that the kernel takes
+    s1, with_ = bytes_of(nodes, "depth 7 persist 1")
+    s1.close()
+    s0, without = bytes_of(nodes, "depth 7 persist 0")
+    s0.close()
+    n = nodes[0] * nodes[1]
+    assert with_ - without < (n // 4 + n // 16 + n // 64) * 1.1 * (9 * 8 + 2)
