@@ -361,14 +361,19 @@ inline int device_sms() {
 }
 
 // Blocks of the whole-GPU kernel when `beside` particles are still being
-// written (the fused step's second pass): a block takes its SM, so the pass
-// goes on with the others, and the best share is the one whose solve ends
-// with the pass.  Steps of 512 particles per row (1025^2 nodes): 9.15 ms with
-// every SM, 8.78 with a quarter, 9.38 with 20 blocks; of 32 per row (128^3):
-// 6.6 ms with every SM, 6.5 with two thirds, 8.3 with a quarter.
+// written (the fused step's second pass): a block takes its SM, so a pass
+// that lasts as long as the solve goes on with the others.  By particles per
+// row; a step with every SM against the share taken from there on:
+//   128^3 rows: 0.01 4.05 / 4.66 ms, 1 6.49 / 7.03, 4 6.46 / 6.66,
+//     16 6.35 / 6.36, 60 8.42 / 8.22 (two thirds; 32 and a quarter: 8.3);
+//   64^3 rows: 8 2.11 / 2.08, 32 2.15 / 2.10, 120 3.14 / 3.03 (two thirds),
+//     500 8.59 / 8.23 (a quarter);
+//   351^2 rows: 64 1.44 / 1.41, 250 1.40 / 1.31 (two thirds),
+//     500 1.89 / 1.71, 1000 3.36 / 2.97 (a quarter);
+//   1025^2 rows: 512 9.15 / 8.78 (a quarter; 20 blocks: 9.38).
 inline int persist_blocks(long long beside, long long rows) {
     const int sms = device_sms();
-    if (beside <= 0) return sms;
+    if (beside < 8 * rows) return sms;
     return std::max(1, beside >= 256 * rows ? sms / 4 : sms * 2 / 3);
 }
 

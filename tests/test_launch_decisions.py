@@ -68,7 +68,7 @@ def test_whole_gpu_cycle_refused(fake, kind, options, how):
     """The same for the kernel of a cycle's coarse levels, in the solve's graph (refused when it is instantiated) and
     launched on a stream that takes no graph."""
     fake.lib.fake_refuse_cooperative(how)
-    s = F.Solver(fake, kind, (64, 64, 272), "tma_min_rows 1000000 " + options)
+    s = F.Solver(fake, kind, (64, 64, 272), "depth 4 tma_min_rows 1000000 " + options)
     s.set_source(np.array([7]), np.array([1.0]))
     fake.lib.fake_clear_log()
     st = fake.stream() if how == 2 else C.c_void_p(1)   # 1: the legacy default stream
@@ -83,7 +83,7 @@ def test_whole_gpu_cycle_refused(fake, kind, options, how):
 
 
 @pytest.mark.parametrize("kind,nodes,options,one_kernel", [
-    (M32, (400, 410), "tol 1e-9", False), (M64, (400, 410), "", False), (M32, (64, 64, 272), "tol 1e-9 tma_min_rows 1000000", False),
+    (M32, (400, 410), "tol 1e-9", False), (M64, (400, 410), "", False), (M32, (64, 64, 272), "depth 4 tol 1e-9 tma_min_rows 1000000", False),
     (M64, (64, 64), "", True), (M32, (96, 96), "tol 1e-9", True)])
 def test_solve_captured_by_the_caller(fake, kind, nodes, options, one_kernel):
     """The caller may replay its graphs beside one another and beside direct solves: nothing in them may wait for blocks
@@ -126,10 +126,9 @@ def test_a_stall_is_told_by_the_next_call(fake):
 
 def test_graph_of_a_solve_is_the_same_beside_a_pending_pass(fake):
     """A graph captured while a fused step's second pass is pending is replayed by solves that run alone: its kernels
-    take every SM whatever was pending at the capture.  A whole solve as one kernel is launched each time and leaves
-    SMs to the pass."""
+    take every SM whatever was pending at the capture."""
     nodes = (64, 64, 272)
-    s = F.Solver(fake, M32, nodes, "tma_min_rows 1000000")
+    s = F.Solver(fake, M32, nodes, "depth 4 tma_min_rows 1000000")
     step, close = F.step_context(fake, tuple(k - 1 for k in nodes), n=1000)
     assert step(s) == 0 and step(s) == 0
     s.set_options("K 272 max_cycles 2")   # the graph is captured again, beside the pending pass
@@ -140,14 +139,19 @@ def test_graph_of_a_solve_is_the_same_beside_a_pending_pass(fake):
     assert {q.grid for q in fake.kernels("k_mg_persist") if q.captured != 1} == {148}
     close()
     s.close()
-    one = F.Solver(fake, M32, (401, 401))
-    step, close = F.step_context(fake, (400, 400), n=1000)
+
+
+@pytest.mark.parametrize("per_row,blocks", [(0.01, 148), (7.9, 148), (8, 98)])
+def test_share_of_the_gpu_beside_a_pending_pass(fake, per_row, blocks):
+    """A whole solve leaves SMs to the pending second pass where that lasts; a short one (few particles per row) would
+    not use them."""
+    s = F.Solver(fake, M32, (331, 331))
+    step, close = F.step_context(fake, (330, 330), n=int(per_row * 331 * 331 + 1))
     fake.lib.fake_clear_log()
-    assert step(one) == 0 and step(one) == 0
-    a, b = (q.grid for q in fake.kernels("k_mg_persist"))
-    assert a == 148 > b
+    assert step(s) == 0 and step(s) == 0
+    assert [q.grid for q in fake.kernels("k_mg_persist")] == [148, blocks]   # nothing is pending at the first
     close()
-    one.close()
+    s.close()
 
 
 def test_tables_only_where_a_kernel_reads_them(fake):
