@@ -179,7 +179,10 @@ __device__ __forceinline__ T exception_row(const PersistStencil<T>& P, const Ite
     if (!P.csr || !__ldg(P.csr + q)) {
         const T* c = P.dense + (long long)q * NS;
 #pragma unroll
-        for (int t = 0; t < NS; ++t) s += __ldg(c + t) * v[t];
+        for (int t = 0; t < NS; ++t) {
+            const T ct = __ldg(c + t);
+            if (ct != T(0)) s += ct * v[t];   // the row has no such tap: 0 times an infinite value is not 0
+        }
         return s;
     }
     const int b = __ldg(P.s.exc_ptr + q), e = __ldg(P.s.exc_ptr + q + 1);
