@@ -1377,8 +1377,9 @@ EXPORT int psum_mg_last_stats(psum_field_solver_handle h, int* cycles, int* refi
         const double bn = st.bnorm2 > 0 ? std::sqrt(st.bnorm2) : 1.0;
         if (cycles) *cycles = st.cycles;
         if (refinements) *refinements = st.refinements;
-        if (rel_residual) *rel_residual = std::sqrt(std::max(0.0, st.rnorm2_last)) / bn;
-        if (initial_rel_residual) *initial_rel_residual = std::sqrt(std::max(0.0, st.rnorm2_first)) / bn;
+        auto rel = [&](double r2) { return r2 < 0 ? 0.0 : std::sqrt(r2) / bn; };   // -1: none was taken; NaN stays NaN
+        if (rel_residual) *rel_residual = rel(st.rnorm2_last);
+        if (initial_rel_residual) *initial_rel_residual = rel(st.rnorm2_first);
     });
 }
 

@@ -32,3 +32,12 @@ def test_infinite_guess_at_a_fixed_node(kind, nodes, node):
     one, many = (outcome(kind, nodes, f"persist {p}", node, math.inf) for p in (1, 0))
     assert one == many
     assert one[0] == 5 and one[1]["rel_residual"] == math.inf
+
+
+@pytest.mark.parametrize("kind", BACKENDS)
+@pytest.mark.parametrize("persist", [1, 0])
+def test_nan_residual_is_told(kind, persist):
+    """A residual that is no number is read as one that is none (the adjoint's convergence check asks whether it is
+    finite), not as zero."""
+    code, stats = outcome(kind, (33, 41), f"persist {persist}", 500, math.nan)
+    assert code == 5 and math.isnan(stats["rel_residual"]) and math.isnan(stats["initial_rel_residual"])
