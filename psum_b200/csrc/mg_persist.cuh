@@ -33,15 +33,16 @@
 
 namespace psum_b200 {
 
-// Threads per block (80 and 128 registers a thread): a 27-point FP64 row keeps
-// twice the registers in flight.
+// Threads per block: a 27-point FP64 row keeps twice the registers in flight.
+// All stencil shapes share a kernel, so it has 80 (FP32) and 128 (FP64)
+// registers a thread and spills 140-200 and 644 bytes at its largest shape.
 template <class T>
 constexpr int kPersistThreads = sizeof(T) == 4 ? 768 : 512;
 constexpr int kPersistLevels = 12;
 constexpr int kClusterBlocks = 16;
 constexpr int kNormVBlocks = 444;           // the fixed grid of the norms: 444 blocks of 256 rows per stride
 constexpr int kNormVWarps = kNormVBlocks * 8;
-constexpr int kBarrierPolls = 1 << 22;      // about 4 s
+constexpr int kBarrierPolls = 1 << 22;      // seconds; a step takes microseconds
 constexpr int kDenseTailRows = 128;         // coarse systems up to this size are solved by the tail's block
 
 enum PersistSync { kSyncBlock = 0, kSyncCluster = 1, kSyncGrid = 2 };
@@ -112,13 +113,11 @@ struct PersistArgs {
 };
 
 // Barrier over the kernel's blocks; every thread calls it.
-template <int SYNC>
+template <int SYNC, class T>
 struct Barrier {
-    unsigned* counter;
-    Stall* stall;
-    int polls;
-    unsigned target = 0;
-    bool broken = false;
+    const PersistArgs<T>& p;
+    unsigned& target;       // thread 0's, in shared memory: every thread would hold a register for it
+    bool& broken;
 
     __device__ __forceinline__ void operator()() {
         if constexpr (SYNC == kSyncBlock) {
@@ -128,17 +127,17 @@ struct Barrier {
         } else {
             __syncthreads();
             if (threadIdx.x == 0) {
-                target += gridDim.x;
-                asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(counter) : "memory");
+                const unsigned want = target += gridDim.x;
+                asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p.counter) : "memory");
                 if (!broken) {
                     unsigned v = 0;
                     int it = 0;
                     for (;;) {
-                        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(counter) : "memory");
-                        if ((int)(v - target) >= 0) break;
-                        if (++it >= polls) {
+                        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p.counter) : "memory");
+                        if ((int)(v - want) >= 0) break;
+                        if (++it >= p.polls) {
                             broken = true;
-                            record_stall(stall);
+                            record_stall(&p.st->stall);
                             break;
                         }
                     }
@@ -179,11 +178,9 @@ __device__ __forceinline__ T exception_row(const PersistStencil<T>& P, const Ite
     if (!P.csr || !__ldg(P.csr + q)) {
         const T* c = P.dense + (long long)q * NS;
 #pragma unroll
-        for (int t = 0; t < NS; ++t) {
-            const T ct = __ldg(c + t);
-            if (ct != T(0)) s += ct * v[t];   // the row has no such tap: 0 times an infinite value is not 0
-        }
-        return s;
+        for (int t = 0; t < NS; ++t) s += __ldg(c + t) * v[t];
+        if (s == s) return s;   // else the row may not have a tap whose value is infinite (0 times that is NaN)
+        s = T(0);
     }
     const int b = __ldg(P.s.exc_ptr + q), e = __ldg(P.s.exc_ptr + q + 1);
 #pragma unroll 1
@@ -728,8 +725,14 @@ __global__ void __launch_bounds__(kPersistThreads<T>, 1) k_mg_persist(const __gr
     extern __shared__ __align__(16) unsigned char persist_smem[];
     __shared__ __align__(16) unsigned char level_smem[sizeof(PersistLevel<T>) * kPersistLevels];
     if (p.mode == kPersistCycle && p.gated && p.st->done) return;
-    Barrier<SYNC> sync{p.counter, &p.st->stall, p.polls};
-    Barrier<kSyncBlock> bsync{nullptr, nullptr, 0};
+    __shared__ unsigned barrier_target;
+    __shared__ bool barrier_broken;
+    if (threadIdx.x == 0) {
+        barrier_target = 0;
+        barrier_broken = false;
+    }
+    Barrier<SYNC, T> sync{p, barrier_target, barrier_broken};
+    Barrier<kSyncBlock, T> bsync{p, barrier_target, barrier_broken};
     const int tid = blockIdx.x * NT + threadIdx.x, nthr = gridDim.x * NT;
     const int warp = tid >> 5, nwarps = nthr >> 5;
     const int n = (int)p.a0.s.n;

@@ -1496,9 +1496,9 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_hist(RsSource a, long long n,
 // its own digit counters (no block barrier), one block scan places the
 // digits, the pairs are put in order in shared memory, and then leave it
 // digit by digit, so that neighbouring threads write neighbouring words.
-// The nine passes of a
-// load, sort and bin of 16.8M particles on a B200: 162 -> 128 us each against
-// a scatter straight from registers with four block barriers per 256 items.
+// 16.8M particles: 187 us the first pass of a random order, 108-117 us the
+// later ones (128 us on average; straight from registers with four block
+// barriers per 256 items: 162 us).
 template <bool RAW>
 __global__ void __launch_bounds__(kRsThreads) k_rs_scatter(RsSource a, unsigned* __restrict__ kout,
                                                            int* __restrict__ vout, long long n, int shift, unsigned mask,
@@ -1671,8 +1671,8 @@ __global__ void __launch_bounds__(256) k_gather_all(GatherSet g, const int* __re
 
 __global__ void k_set_count(long long* count, long long v) { *count = v; }
 
-// Valid particles (keys >= 0) of a state: one read of the keys (67 MB in
-// 20 us at 16.8M particles; copied to the host and counted there it took 38 ms).
+// Valid particles (keys >= 0) of a state: one read of the keys, bound by it
+// (67 MB in 20 us at 16.8M particles; counting a host copy: 38 ms).
 __global__ void __launch_bounds__(256) k_count_keys(const int* __restrict__ key, long long n,
                                                     unsigned long long* __restrict__ out) {
     unsigned v = 0;
