@@ -339,9 +339,13 @@ void launch_residual64(const StencilDev<double>& A, const double* x, const doubl
 // Which levels one kernel takes, and how its blocks meet.  Solves on a B200,
 // one launch per step against one kernel: 64^2 FP64 3.3 -> 0.43 ms, 256^2
 // mixed 4.4 -> 0.63, 1025^2 mixed 6.0 -> 1.24, 33 x 41 x 29 FP64 4.3 -> 1.7,
-// 128^3 mixed 7.2 -> 2.3 (14 cycles), 256^3 mixed 17.0 -> 14.1 (coarse levels
-// only; 21.4 with all levels inside: its finest level streams from HBM, where
-// the TMA-staged sweep is twice as fast).
+// 128^3 mixed 7.2 -> 2.3 (14 cycles).  About the limit, to 1e-8: 1400^2 mixed
+// 3.8 -> 2.1, 128^3 FP64 4.9 -> 4.1 (all levels); 1504 x 1600 mixed 3.9 -> 3.7,
+// 2049^2 mixed 5.0 -> 4.1, 129^3 mixed 6.1 -> 4.4, 160^3 mixed 5.7 -> 5.0 and
+// FP64 6.9 -> 6.5, 200^3 mixed 15.0 -> 12.5 (coarse levels only).  256^3 mixed
+// takes 14.1 that way and 21.4 with all levels inside: its finest level
+// streams from HBM, where the TMA-staged sweep is twice as fast.  Finest
+// levels between 2^21 and 2^24 rows were not tried inside the kernel.
 constexpr long long kPersistRows = 1LL << 21;     // largest level worked inside the kernel
 // Up to here one cluster of 16 blocks, above one block per SM: a cluster
 // barrier and its loads take about 1 us a step against 2.6, but 16 SMs sweep
