@@ -35,6 +35,12 @@ unsigned long long thread_launches();   // launches counted by the calling threa
 // conditional graph loop); psum_kernel_launches includes it.
 unsigned long long* device_launch_counter();
 
+// A zeroed pinned, device-mapped word (a kernel's report to the host), from
+// pages of 1024 that the process keeps: pinning a page takes up to
+// milliseconds, and every solver handle needs a word.
+int* take_host_word();
+void give_host_word(int* w);
+
 inline void cuda_check(cudaError_t e, const char* what) {
     if (e != cudaSuccess) throw Error(PSUM_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
 }

@@ -606,7 +606,7 @@ struct SolverBase {
         drop_graph();
         if (aux_stream) cudaStreamDestroy(aux_stream);
         if (own_stream) cudaStreamDestroy(own_stream);
-        if (stalled) cudaFreeHost(stalled);
+        give_host_word(stalled);   // the solver's buffers are freed by now, which waits for its kernels
     }
     void drop_graph() {
         if (graph.exec) cudaGraphExecDestroy(graph.exec);
@@ -1126,12 +1126,7 @@ void solver_set_matrix(SolverBase* s, unsigned long long n_row, unsigned long lo
     // body of the conditional refinement loop, and the mapped launch counter
     if (!s->aux_stream) cuda_check(cudaStreamCreateWithFlags(&s->aux_stream, cudaStreamNonBlocking), "cudaStreamCreate");
     device_launch_counter();
-    if (!s->stalled) {
-        void* p = nullptr;
-        cuda_check(cudaHostAlloc(&p, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable), "cudaHostAlloc stall word");
-        s->stalled = static_cast<int*>(p);
-        *s->stalled = 0;
-    }
+    if (!s->stalled) s->stalled = take_host_word();
     s->version++;
     s->drop_graph();
     s->build_device(s->own_stream);

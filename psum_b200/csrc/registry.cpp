@@ -9,6 +9,7 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <vector>
 
 #include "common.hpp"
 
@@ -39,6 +40,38 @@ unsigned long long* device_launch_counter() {
         g_mapped = static_cast<unsigned long long*>(p);
     });
     return g_mapped;
+}
+
+namespace {
+struct HostWords {
+    std::mutex m;
+    std::vector<int*> free;
+};
+HostWords& host_words() {
+    static HostWords* w = new HostWords;   // never destroyed: a handle may outlive the statics
+    return *w;
+}
+}  // namespace
+
+int* take_host_word() {
+    HostWords& h = host_words();
+    std::lock_guard<std::mutex> lk(h.m);
+    if (h.free.empty()) {
+        constexpr int kPage = 1024;
+        void* p = nullptr;
+        cuda_check(cudaHostAlloc(&p, kPage * sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable), "cudaHostAlloc");
+        for (int i = kPage - 1; i >= 0; --i) h.free.push_back(static_cast<int*>(p) + i);
+    }
+    int* w = h.free.back();
+    h.free.pop_back();
+    *static_cast<volatile int*>(w) = 0;
+    return w;
+}
+void give_host_word(int* w) {
+    if (!w) return;
+    HostWords& h = host_words();
+    std::lock_guard<std::mutex> lk(h.m);
+    h.free.push_back(w);
 }
 
 void count_launch() {

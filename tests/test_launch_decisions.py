@@ -109,18 +109,19 @@ def test_solve_captured_by_the_caller(fake, kind, nodes, options, one_kernel):
 
 def test_a_stall_is_told_by_the_next_call(fake):
     """The pinned word that a kernel sets when it gives up a wait reaches the caller whichever call comes next, once."""
-    before = fake.pinned_words()
     s = F.Solver(fake, M32, (33, 33))
-    (word,) = fake.pinned_words() - before
-    word = C.c_int.from_address(word)
     step, close = F.step_context(fake, (32, 32))
     st = fake.stream()
     for call in (s.solve, lambda: s.solve_async(st), s.last_stats, lambda: step(s)):
         assert call() == 0
-        word.value = 1
+        fake.set_host_words(1)
         assert call() == 8 and b"stopped waiting" in fake.lib.psum_last_error()
         assert call() == 0
     close()
+    fake.set_host_words(1)
+    s.close()
+    s = F.Solver(fake, M32, (33, 33))   # the word of a handle that is gone
+    assert s.solve() == 0
     s.close()
 
 
