@@ -110,7 +110,7 @@ API unsigned long long fake_device_bytes() {
     for (auto& m : device_mem) b += m.second;
     return b;
 }
-// The live pinned host blocks of a size, newest address last in `out`; returns how many there are.
+// The live pinned host blocks of a size; returns how many there are.
 API int fake_pinned(unsigned long long bytes, void** out, int cap) {
     int n = 0;
     for (auto& m : host_mem)
